@@ -71,7 +71,7 @@ def parse():
                     help="arrival rates [jobs/s] of the served sweep")
     ap.add_argument("--sweep-seconds", type=float, default=4.0, help="length of each trace of the served sweep")
     ap.add_argument("--profile-job", choices=["active", "dense", "mc", "mcfull"], default=None,
-                    help="run exactly one CA job with this schedule (no warm-up, no MC), or with mc one ACTIVE "
+                    help="run exactly one CA job with this schedule (active: the tile list; no warm-up, no MC), or with mc one ACTIVE "
                          "CA job and its MC stage, or with mcfull the whole-space MC case (--max-steps sweeps), "
                          "and exit: the case ncu captures")
     ap.add_argument("--max-steps", type=int, default=None, help="with --profile-job: stop the CA after this many steps")
@@ -599,19 +599,20 @@ def ours(args):
     attempts = sum(j["mc"]["attempts"] for j in jobs)
     launches = sum(j["launches"] + j["mc"]["launches"] for j in jobs)
 
-    # the same job with the DENSE schedule, and profiled jobs (per-kernel CUDA events) of both schedules
+    # the same job with the DENSE schedule, and profiled jobs (per-kernel CUDA events) of the tile kernels' two
+    # schedules (the default ACTIVE schedule is one launch per 64 steps and has no per-step kernels)
     dense = Resident(w, capi.SWEEP_DENSE, local)
     dj = dense.run(flush, mc=False)
     dense.close()
     profs = {}
-    for name, sweep in (("active", capi.SWEEP_ACTIVE), ("dense", capi.SWEEP_DENSE)):
+    for name, sweep in (("active_list", capi.SWEEP_ACTIVE_LIST), ("dense", capi.SWEEP_DENSE)):
         pr = Resident(w, sweep, local, profile=True)
         pj = pr.run(flush, mc=False)
         pj["kernels"] = pr.ca.kernel_times()
         pr.close()
         profs[name] = pj
     roof_dense = roofline(profs["dense"], w, "dense", peak, peak_kind)
-    roof_active = roofline(profs["active"], w, "active", peak, peak_kind)
+    roof_active = roofline(profs["active_list"], w, "active", peak, peak_kind)
 
     # e2e through the C ABI with host buffers on resident handles: two jobs in flight (one computing,
     # one copying), and one at a time
@@ -663,7 +664,7 @@ def ours(args):
         "vs_baseline": None, "dtype": "u8+i32+f32 (integer rules, f32 temperatures)",
         "data": "synthetic (seeded Gaussian-cone terrain written as the reference's CSV heightmap)",
         "config": config_of(w),
-        "method": {"schedule": "ACTIVE (tile skipping, bit-identical to DENSE)",
+        "method": {"schedule": "ACTIVE (list of LAVA cells, bit-identical to DENSE)",
                    "l2": "flushed (256 MiB write) before every CA run and MC run, outside their device events; "
                          "the state (13 B x 2 buffers per cell) is far larger than L2",
                    "timing": "CUDA events on the handle's stream around the step launches of each job",
@@ -676,9 +677,9 @@ def ours(args):
         "dense": {"value": world * w.cells * dj["steps"] / (dense_ms * 1e-3), "ms_per_step": dense_ms},
         "roofline": roof_dense,
         "roofline_active": roof_active,
-        "kernels_ms": {"active": profs["active"]["kernels"], "dense": profs["dense"]["kernels"]},
-        "active_tiles_frac": round(profs["active"]["tiles"] / max(1, profs["active"]["tiles_total"] *
-                                                                   profs["active"]["steps"]), 4),
+        "kernels_ms": {"active_list": profs["active_list"]["kernels"], "dense": profs["dense"]["kernels"]},
+        "active_tiles_frac": round(profs["active_list"]["tiles"] / max(1, profs["active_list"]["tiles_total"] *
+                                                                   profs["active_list"]["steps"]), 4),
         "e2e": {"value": world * w.cells * e2e_steps / (e2e_ms * 1e-3), "unit": "cell-updates/s",
                 "h2d_bytes_per_step": e2e_h2d, "d2h_bytes_per_step": e2e_d2h, "ms_per_step": e2e_ms / e2e_jobs,
                 "jobs": e2e_jobs, "jobs_in_flight": E2E_INFLIGHT, "phases_median": e2e_phases,
@@ -761,7 +762,7 @@ def profile_job(args):
     w = workloads.get(args.workload)
     if args.max_steps is not None:
         w.max_steps = args.max_steps
-    sweep = capi.SWEEP_DENSE if args.profile_job == "dense" else capi.SWEEP_ACTIVE
+    sweep = capi.SWEEP_DENSE if args.profile_job == "dense" else capi.SWEEP_ACTIVE_LIST
     ca = capi.LavaCA(ca_params(w, sweep, 0))
     ca.apply_terrain(w.heights)
     ca.place_seeds(w.vent_cells())

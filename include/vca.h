@@ -44,10 +44,11 @@ enum { VCA_BC_ABSORBING = 0, VCA_BC_PERIODIC = 1 };
 enum { VCA_MODE_LAVA = 0, VCA_MODE_CLASSIC = 1 };
 /* Step schedule.  All give bit-identical results (grids, histories, stop step), like the
  * reference's ca.sweep = front / full (engine/src/ca/LavaCA.hpp:13-29):
- *   ACTIVE      -- tiles with no lava within one cell, and unchanged since the last step, are
- *                  skipped; a grid whose every tile has a rules block of its own runs DENSE;
+ *   ACTIVE      -- only the LAVA cells and the AIR cells they reach, from a list of the LAVA cells
+ *                  (nothing else can change in a step);
  *   DENSE       -- every cell of the grid is read and written every step;
- *   ACTIVE_LIST -- ACTIVE with the tile list whatever the grid size. */
+ *   ACTIVE_LIST -- tiles with no lava within one cell, and unchanged since the last step, are
+ *                  skipped. */
 enum { VCA_SWEEP_ACTIVE = 0, VCA_SWEEP_DENSE = 1, VCA_SWEEP_ACTIVE_LIST = 2 };
 /* StopReason (engine/src/ca/CaRules.hpp:108) */
 enum { VCA_STOP_RUNNING = 0, VCA_STOP_NO_LAVA = 1, VCA_STOP_NO_AIR = 2, VCA_STOP_NO_CHANGE = 3,
@@ -103,7 +104,8 @@ typedef struct {
     uint64_t lava_cells;       /* LAVA cells now (classic: grains) */
     uint64_t air_cells;        /* AIR cells now */
     uint64_t tiles_total;      /* tiles of the grid */
-    uint64_t tiles_processed;  /* tile visits summed over all steps (DENSE: steps x tiles) */
+    uint64_t tiles_processed;  /* tile visits summed over all steps (DENSE: steps x tiles; ACTIVE: its visits
+                                * of LAVA cells, in tiles of cells_per_tile) */
     uint64_t cells_per_tile;   /* cells one tile covers */
     uint64_t kernel_launches;  /* CUDA kernel launches issued by this handle so far */
 } vca_ca_info;
@@ -187,11 +189,12 @@ vca_status vca_ca_layers(vca_ca* ca, void** type, void** flow_id, void** temp, v
 vca_status vca_ca_pack_layers(vca_ca* ca, int z0, int types, int full, void* buf);
 vca_status vca_ca_unpack_layers(vca_ca* ca, int z0, int types, int full, const void* buf);
 /* Device time of the CA steps so far [ms] (CUDA events around the step launches) and the average
- * duration of one launch of the rules kernel [ms] over the last vca_ca_run / vca_ca_step calls. */
+ * duration of one launch of the rules kernel [ms] (handles created with VCA_PROFILE_KERNELS=1). */
 vca_status vca_ca_timing(vca_ca* ca, double* total_ms, double* rules_kernel_ms, uint64_t* rules_launches);
 /* With VCA_PROFILE_KERNELS=1 in the environment when the handle was created, runs launch step by
- * step with CUDA events around each kernel: the average device time [ms] of the drop-depth, rules
- * and candidate kernels of a step, and the steps measured.  No counterpart in the reference. */
+ * step with CUDA events around each kernel (an ACTIVE handle then steps as ACTIVE_LIST): the average
+ * device time [ms] of the drop-depth, rules and candidate kernels of a step, and the steps measured.
+ * No counterpart in the reference. */
 vca_status vca_ca_kernel_times(vca_ca* ca, double* drop_ms, double* rules_ms, double* cand_ms, uint64_t* steps);
 /* ~LavaCA: frees the handle's device memory, stream and graph. */
 void vca_ca_destroy(vca_ca* ca);
@@ -200,9 +203,9 @@ void vca_ca_destroy(vca_ca* ca);
  * Batched stepping of many lava CA grids.  No counterpart in the reference: its batch runner
  * (engine/src/app/Batch.cpp:186-246) starts one engine process per config, one after another, and
  * each LavaCA::run (LavaCA.hpp:253-256) steps one grid.  A batch steps every member grid -- of any
- * size, 2D or 3D, neighbourhood, boundary, seed or schedule -- with three launches per step for all
- * of them together (each block of a launch works on one member), captured as a CUDA graph of 16
- * steps.  Each member ends exactly as it would alone (same planes, histories and stop step).
+ * size, 2D or 3D, neighbourhood, boundary, seed or schedule -- with shared launches (each block of a
+ * launch works on one member): one launch of 16 steps for the ACTIVE members, three launches per
+ * step, captured as a CUDA graph of 16 steps, for the others.  Each member ends exactly as it would alone (same planes, histories and stop step).
  * ---------------------------------------------------------------------------------------- */
 
 /* A batch of at most max_members grids on a device (max_members is also capped by the blocks of
@@ -213,8 +216,8 @@ vca_status vca_ca_batch_create(int device, int max_members, vca_ca_batch** out);
  * rule holds (vca_ca_batch_advance reports it) or by vca_ca_batch_remove.  VCA_ERR_ARG when the
  * batch is full or the handle lives on another device or in another batch. */
 vca_status vca_ca_batch_add(vca_ca_batch* b, vca_ca* member);
-/* Steps the members: launches up to max_graphs graphs of 16 steps, reading each graph's stop flags
- * while the next one runs, and returns once some member has stopped (or all graphs are done, or no
+/* Steps the members: launches up to max_graphs rounds of 16 steps, reading each round's stop flags
+ * while the next one runs, and returns once some member has stopped (or all rounds are done, or no
  * member is left).  The members that stopped leave the batch and are written to finished[0..*count)
  * (at most capacity; the others stay queued for the next call); running gets the members still
  * stepping.  A member that had stopped before it was added is reported by the next call. */
@@ -222,7 +225,7 @@ vca_status vca_ca_batch_advance(vca_ca_batch* b, int max_graphs, vca_ca** finish
                                 int* running);
 /* Takes a member out of the batch now, whatever its state (its last step completes first). */
 vca_status vca_ca_batch_remove(vca_ca_batch* b, vca_ca* member);
-/* Launch counts: graphs launched, kernel launches issued, members now. */
+/* Launch counts: rounds of 16 steps launched, kernel launches issued, members now. */
 vca_status vca_ca_batch_info(vca_ca_batch* b, uint64_t* graphs, uint64_t* launches, int* members);
 /* Detaches every member (as by vca_ca_batch_remove) and frees the batch. */
 void vca_ca_batch_destroy(vca_ca_batch* b);

@@ -1,4 +1,5 @@
-// ca.cu -- lava cellular automaton on sm_100a: kernels and the vca_ca_* half of the C ABI.
+// ca.cu -- lava cellular automaton on sm_100a: the tile kernels (DENSE and ACTIVE_LIST schedules, z
+// slabs; the ACTIVE schedule is stepped by front.cu) and the vca_ca_* half of the C ABI.
 //
 // One CA step (LavaCA::step, engine/src/ca/LavaCA.hpp:230-247) is three launches on the handle's
 // stream:
@@ -16,7 +17,7 @@
 // in pitched rows; the current buffer is the parity of the device-side step counter, so a run of
 // steps needs no host round trip until the stop test.
 //
-// ACTIVE schedule: only LAVA cells and AIR cells with LAVA within one cell can change in a step
+// ACTIVE_LIST schedule: only LAVA cells and AIR cells with LAVA within one cell can change in a step
 // (the front set of LavaCA::frontCandidatesLayer, LavaCA.hpp:907-940).  A tile is processed in step
 // t+1 when a tile within one tile of it holds LAVA after step t, or when it changed in step t (its
 // two buffers then differ).  Every other tile keeps both buffers equal and is skipped; the result is
@@ -34,6 +35,7 @@
 #include <utility>
 #include <vector>
 
+#include "ca_cells.cuh"
 #include "vca.h"
 #include "vca_device.cuh"
 #include "vca_internal.h"
@@ -42,151 +44,8 @@ namespace vca {
 
 constexpr int kThreads = 256;       // threads of a tile block: 16 per 64-cell row, 16 rows
 constexpr int kTileX = 64;
-constexpr int kMaxDrop = 16;        // LavaCA::kMaxDrop (LavaCA.hpp:1293)
 constexpr int kSmemRowBytes = 96;   // 16 pad (left frame byte at 15) + 64 cells + right frame byte + pad
 constexpr int kRowOff = 16;         // first cell of a staged row (16-byte aligned for cp.async)
-
-// ------------------------------------------------------------------------------------------
-// Addressing with the reference's frame semantics: a coordinate one step outside the interior is
-// the opposite layer on a periodic axis, else the VOID frame (Boundary::applyWith,
-// engine/src/core/Boundary.hpp:75-131).
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ int64_t pidx(const CaGeom& g, int x, int y, int z) {
-    return (int64_t)x + (int64_t)g.P * ((int64_t)y + (int64_t)g.ny * z);
-}
-__device__ __forceinline__ bool wrap_axis(int& v, int n, int periodic) {
-    if (v >= 0 && v < n) return true;
-    if (!periodic || n == 1) return false;
-    v = v < 0 ? v + n : v - n;
-    return true;
-}
-__device__ __forceinline__ bool resolve(const CaGeom& g, int& x, int& y, int& z) {
-    return wrap_axis(x, g.nx, g.per[0]) && wrap_axis(y, g.ny, g.per[1]) && wrap_axis(z, g.nz, g.per[2]);
-}
-// A halo coordinate of a tile: up to one cell outside [0, n) maps through the frame; further out
-// (past a partial last tile) is outside the grid.
-__device__ __forceinline__ bool halo_axis(int& v, int n, int periodic) {
-    if (v > n) return false;
-    return wrap_axis(v, n, periodic);
-}
-__device__ __forceinline__ bool solid_ground(int t) { return t == kRock || t == kBasalt; }
-// resolve() for a neighbour one cell away, as selects instead of branches, so that the loads of
-// all neighbours of a cell can be issued together.  v is only meaningful when the result is true.
-__device__ __forceinline__ bool wrap1_sel(int& v, int n, int periodic) {
-    const bool in = (unsigned)v < (unsigned)n;
-    const int w = v < 0 ? v + n : v - n;
-    v = in ? v : w;
-    return in | ((periodic != 0) & (n > 1));
-}
-__device__ __forceinline__ bool resolve1_sel(const CaGeom& g, int& x, int& y, int& z) {
-    const bool a = wrap1_sel(x, g.nx, g.per[0]), b = wrap1_sel(y, g.ny, g.per[1]), c = wrap1_sel(z, g.nz, g.per[2]);
-    return a & b & c;
-}
-
-// CandidateVote (engine/src/ca/CaRules.hpp:127-183).
-struct Vote {
-    int n;
-    int32_t ids[26];
-    int counts[26];
-    float max_temp[26];
-    __device__ void add(int32_t id, float t) {
-        for (int i = 0; i < n; ++i)
-            if (ids[i] == id) {
-                ++counts[i];
-                max_temp[i] = fmaxf(max_temp[i], t);
-                return;
-            }
-        ids[n] = id;
-        counts[n] = 1;
-        max_temp[n] = t;
-        ++n;
-    }
-    // Most votes; ties: tied ids ascending, pick hashRand(seed, t, idx, TieBreak) % k.
-    __device__ int winner(uint64_t prefix, uint64_t gidx) const {
-        if (n == 1) return 0;
-        int best = 0;
-        for (int i = 0; i < n; ++i) best = max(best, counts[i]);
-        int tied[26];
-        int k = 0;
-        for (int i = 0; i < n; ++i)
-            if (counts[i] == best) tied[k++] = i;
-        if (k == 1) return tied[0];
-        for (int i = 1; i < k; ++i) {
-            const int t = tied[i];
-            int j = i;
-            while (j > 0 && ids[tied[j - 1]] > ids[t]) {
-                tied[j] = tied[j - 1];
-                --j;
-            }
-            tied[j] = t;
-        }
-        const uint64_t r = hash_salt(hash_index(prefix, gidx), kSaltTieBreak);
-        return tied[(int)(r % (uint64_t)k)];
-    }
-    __device__ bool overflow() const { return false; }
-    __device__ void pick(uint64_t prefix, uint64_t gidx, int32_t* id, float* t) const {
-        const int w = winner(prefix, gidx);
-        *id = ids[w];
-        *t = max_temp[w];
-    }
-};
-
-// The same vote for up to 4 distinct flowIds, held in registers (every index is a compile-time
-// constant after unrolling).  A fifth distinct id sets overflow; the caller then recounts with Vote.
-struct SmallVote {
-    int n;
-    bool over;
-    int32_t ids[4];
-    int counts[4];
-    float max_temp[4];
-    __device__ void add(int32_t id, float t) {
-        bool hit = false;
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-            if (s < n && ids[s] == id) {
-                ++counts[s];
-                max_temp[s] = fmaxf(max_temp[s], t);
-                hit = true;
-            }
-        if (hit) return;
-        if (n == 4) {
-            over = true;
-            return;
-        }
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-            if (s == n) {
-                ids[s] = id;
-                counts[s] = 1;
-                max_temp[s] = t;
-            }
-        ++n;
-    }
-    __device__ bool overflow() const { return over; }
-    // Most votes; ties: the (r % k)-th smallest tied id, r = hashRand(seed, t, idx, TieBreak).
-    __device__ void pick(uint64_t prefix, uint64_t gidx, int32_t* id, float* t) const {
-        int best = 0;
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-            if (s < n) best = max(best, counts[s]);
-        int k = 0;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) k += (s < n && counts[s] == best) ? 1 : 0;
-        int want = 0;
-        if (k > 1) want = (int)(hash_salt(hash_index(prefix, gidx), kSaltTieBreak) % (uint64_t)k);
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            if (!(s < n && counts[s] == best)) continue;
-            int rank = 0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) rank += (u < n && counts[u] == best && ids[u] < ids[s]) ? 1 : 0;
-            if (rank == want) {
-                *id = ids[s];
-                *t = max_temp[s];
-            }
-        }
-    }
-};
 
 __device__ __forceinline__ void tile_origin(const CaGeom& g, uint32_t tile, int& x0, int& y0, int& z0) {
     uint32_t tx, ty;
@@ -561,22 +420,6 @@ __device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.w
 
 // Shared-memory row of the tile cell (ly, lz) in the staged halo layout.
 __device__ __forceinline__ int hr_of(int ly, int lz, int hy_on, int hz_on, int HY) { return (ly + hy_on) + HY * (lz + hz_on); }
-
-// Warp-aggregated append of n entries (values v[0..n-1], n <= 4) per lane to list/count.
-__device__ __forceinline__ void warp_append(uint32_t* list, unsigned int* count, uint32_t cap, int lane, unsigned n,
-                                            const uint32_t* v) {
-    unsigned incl = n;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const unsigned u = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-        if (lane >= off) incl += u;
-    }
-    unsigned base = 0;
-    if (lane == 31 && incl) base = atomicAdd(count, incl);
-    base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - n;
-    for (unsigned j = 0; j < n; ++j)
-        if (base + j < cap) list[base + j] = v[j];
-}
 
 constexpr int kMaxDeferred = 64;   // tiles a rules block schedules in one batch
 constexpr int kTileCells = 1024;   // 64 x TY x TZ, TY * TZ = 16
@@ -1551,10 +1394,8 @@ struct CaBatchView {
     const CaKernelArgs* args;  // per member slot
     const int2* rules_map;     // per block of the drop / rules launches: (slot, block within the member)
     const int2* cand_map;      // per block of the candidate launch
-    const int* rules_n;        // per slot: its blocks in the drop / rules launches (0: free slot)
+    const int* rules_n;        // per slot: its blocks in the drop / rules launches (0: not stepped by them)
     const int* cand_n;         // per slot: its blocks in the candidate launch
-    int4* status;              // per slot after a graph: (stop, error, steps, next tiles) or (-1, 0, 0, 0)
-    int slots;
 };
 
 __device__ __forceinline__ void load_args(CaKernelArgs& dst, const CaKernelArgs& src) {
@@ -1597,16 +1438,18 @@ __global__ __launch_bounds__(kCandThreads, 4) void ca_cand_batch_kernel(const __
     cand_body(s_k, (uint32_t)m.y, (uint32_t)b.cand_n[m.x]);
 }
 
-// Stop state of every member after a graph of steps, and the tiles its next step will visit,
-// gathered for one copy to the host.
-__global__ void ca_batch_status_kernel(const __grid_constant__ CaBatchView b) {
-    for (int i = threadIdx.x; i < b.slots; i += blockDim.x) {
+// Stop state of every member after a round of steps and the size of its next one (tiles, or cells of
+// the front list), written into host-mapped memory (a copy would queue behind other handles' downloads
+// on the copy engines).  ctrl: per slot the member's control block (nullptr: free slot).
+__global__ void ca_batch_status_kernel(CaCtrl* const* ctrl, const int* front_n, volatile int* status, int slots) {
+    for (int i = threadIdx.x; i < slots; i += blockDim.x) {
         int4 st = make_int4(-1, 0, 0, 0);
-        if (b.rules_n[i] > 0) {
-            const CaCtrl* c = b.args[i].ctrl;
-            st = make_int4(c->stop, c->error, (int)c->steps, (int)c->list_count[c->steps & 1u]);
-        }
-        b.status[i] = st;
+        if (const CaCtrl* c = ctrl[i])
+            st = make_int4(c->stop, c->error, (int)c->steps, (int)(front_n[i] ? c->front_n : c->list_count[c->steps & 1u]));
+        status[4 * i] = st.x;
+        status[4 * i + 1] = st.y;
+        status[4 * i + 2] = st.z;
+        status[4 * i + 3] = st.w;
     }
 }
 
@@ -1630,19 +1473,31 @@ __global__ void ca_seed_kernel(const __grid_constant__ CaKernelArgs k, const int
 // ============================================================================================
 using namespace vca;
 
+namespace vca {
+// Pull the control block to the host mirror.
+vca_status sync_ctrl(vca_ca* h) {
+    ca_ctrl_snapshot_kernel<<<1, 32, 0, h->stream>>>(h->ctrl, h->ctrl_host_dev);
+    VCA_CUDA(cudaGetLastError());
+    VCA_CUDA(cudaStreamSynchronize(h->stream));
+    h->steps = (int)h->ctrl_host->steps;
+    h->stop = h->ctrl_host->stop;
+    if (h->ctrl_host->error) {
+        set_error("vca_ca: a bounded device wait (TMA tile copy) ran out; the run was stopped");
+        return VCA_ERR_TIMEOUT;
+    }
+    return VCA_OK;
+}
+}  // namespace vca
+
 namespace {
 
-// batched: the arguments of a batch member, whose blocks the batch shares out.  A single grid whose
-// every tile has a rules block of its own runs every tile every step under VCA_SWEEP_ACTIVE (the
-// tile list and its atomics buy nothing there, and the results are the same either way).
-CaKernelArgs make_args(const vca_ca* h, bool batched = false) {
+CaKernelArgs make_args(const vca_ca* h) {
     CaKernelArgs k;
     std::memset(&k, 0, sizeof(k));
     k.g = h->geom;
     k.classic = h->desc.mode == VCA_MODE_CLASSIC;
     k.ponding = h->desc.ponding != 0;
-    k.dense = h->desc.sweep == VCA_SWEEP_DENSE ||
-              (h->desc.sweep == VCA_SWEEP_ACTIVE && !batched && h->ntiles <= (uint64_t)h->grid_blocks);
+    k.dense = h->desc.sweep == VCA_SWEEP_DENSE;
     k.seed = h->desc.seed;
     k.max_steps = h->desc.max_steps;
     k.eruption_steps = h->desc.eruption_steps;
@@ -1716,23 +1571,13 @@ void drop_graph(vca_ca* h) {
     h->graph_exec = nullptr;
 }
 
-// Pull the control block to the host mirror.
-vca_status sync_ctrl(vca_ca* h) {
-    ca_ctrl_snapshot_kernel<<<1, 32, 0, h->stream>>>(h->ctrl, h->ctrl_host_dev);
-    VCA_CUDA(cudaGetLastError());
-    VCA_CUDA(cudaStreamSynchronize(h->stream));
-    h->steps = (int)h->ctrl_host->steps;
-    h->stop = h->ctrl_host->stop;
-    if (h->ctrl_host->error) {
-        set_error("vca_ca: a bounded device wait (TMA tile copy) ran out; the run was stopped");
-        return VCA_ERR_TIMEOUT;
-    }
-    return VCA_OK;
-}
+// Handles with the ACTIVE schedule are stepped by the front kernels (front.cu); the tile kernels step
+// the DENSE and ACTIVE_LIST schedules, slabs, and handles that time each kernel of a step.
+bool wants_front(const vca_ca* h) { return h->desc.sweep == VCA_SWEEP_ACTIVE && !h->slab && !h->profile_kernels; }
 
-// Totals and initial stop state of the current buffer, the first tile list, and a copy of the
-// current buffer into the other one (both buffers equal: the ACTIVE schedule relies on it).
-vca_status init_state(vca_ca* h, int steps_done) {
+// What the tile kernels need besides the planes: a copy of the current buffer in the other one (both
+// buffers equal: the ACTIVE_LIST schedule relies on it), totals, drop depths, the first tile list.
+vca_status tile_init(vca_ca* h, int steps_done) {
     const int cur = steps_done & 1, oth = cur ^ 1;
     const size_t n = h->plane_cells;
     VCA_CUDA(cudaMemcpyAsync(h->type[oth], h->type[cur], n, cudaMemcpyDeviceToDevice, h->stream));
@@ -1742,6 +1587,20 @@ vca_status init_state(vca_ca* h, int steps_done) {
     VCA_CUDA(cudaMemcpyAsync(h->arrival[oth], h->arrival[cur], n * 2, cudaMemcpyDeviceToDevice, h->stream));
     VCA_CUDA(cudaMemsetAsync(h->tile_mark[0], 0, h->ntiles * 4, h->stream));
     VCA_CUDA(cudaMemsetAsync(h->tile_mark[1], 0, h->ntiles * 4, h->stream));
+    CaKernelArgs k = make_args(h);
+    const int blocks = (int)std::min<uint64_t>(h->ntiles, (uint64_t)h->grid_blocks * 4);
+    ca_tile_init_kernel<<<blocks, kThreads, 0, h->stream>>>(k, cur);
+    VCA_CUDA(cudaGetLastError());
+    ca_drop_kernel<<<h->grid_blocks, kThreads, 0, h->stream>>>(k, 1);
+    VCA_CUDA(cudaGetLastError());
+    const int sb = (int)std::min<uint64_t>((h->ntiles + 255) / 256, 4096);
+    ca_init_schedule_kernel<<<sb, 256, 0, h->stream>>>(k, (uint32_t)steps_done);
+    VCA_CUDA(cudaGetLastError());
+    return VCA_OK;
+}
+
+// Totals and initial stop state of the current buffer, and what the handle's step kernels start from.
+vca_status init_state(vca_ca* h, int steps_done) {
     CaCtrl c;
     std::memset(&c, 0, sizeof(c));
     c.steps = (uint32_t)steps_done;
@@ -1749,20 +1608,16 @@ vca_status init_state(vca_ca* h, int steps_done) {
     c.random_nb = h->tables_host.nb.variants > 1;
     c.classic = h->desc.mode == VCA_MODE_CLASSIC;
     VCA_CUDA(cudaMemcpyAsync(h->ctrl, &c, sizeof(c), cudaMemcpyHostToDevice, h->stream));
-    CaKernelArgs k = make_args(h);
-    const int blocks = (int)std::min<uint64_t>(h->ntiles, (uint64_t)h->grid_blocks * 4);
-    ca_tile_init_kernel<<<blocks, kThreads, 0, h->stream>>>(k, cur);
-    VCA_CUDA(cudaGetLastError());
-    ca_drop_kernel<<<h->grid_blocks, kThreads, 0, h->stream>>>(k, 1);
-    VCA_CUDA(cudaGetLastError());
-    {
-        const int sb = (int)std::min<uint64_t>((h->ntiles + 255) / 256, 4096);
-        ca_init_schedule_kernel<<<sb, 256, 0, h->stream>>>(k, (uint32_t)steps_done);
-        VCA_CUDA(cudaGetLastError());
+    if (wants_front(h)) {
+        h->front_buf = h->cur();
+        h->front = true;
+        if (vca_status s = front_init(h, steps_done)) return s;
+    } else {
+        if (vca_status s = tile_init(h, steps_done)) return s;
     }
     if (vca_status s = sync_ctrl(h)) return s;
     CaCtrl* m = h->ctrl_host;
-    const uint64_t lava = m->acc_active, air = m->acc_born;
+    const uint64_t lava = h->front ? m->front_n : m->acc_active, air = m->acc_born;
     m->acc_active = 0;
     m->acc_born = 0;
     m->lava = lava;
@@ -1887,6 +1742,7 @@ vca_status run_steps(vca_ca* h, int max_new_steps, bool until_stop) {
         return VCA_ERR_STATE;
     }
     if (h->stop != VCA_STOP_RUNNING) return VCA_OK;
+    if (h->front) return front_run(h, max_new_steps, until_stop);
     const CaKernelArgs k = make_args(h);
     if (until_stop && !h->profile_kernels) return run_graphs(h, k);
     VCA_CUDA(cudaEventRecord(h->ev_a, h->stream));
@@ -2251,6 +2107,7 @@ vca_status configure(vca_ca* h, const vca_ca_desc* d) {
     if (vca_status s = upload_vents(h, &none, 0)) return s;  // synchronizes the stream
     h->has_terrain = false;
     h->seeded = false;
+    h->front = false;
     h->steps = 0;
     h->stop = VCA_STOP_RUNNING;
     return VCA_OK;
@@ -2389,6 +2246,7 @@ vca_status vca_ca_reset(vca_ca* h) {
     if (vca_status s = upload_vents(h, &none, 0)) return s;  // synchronizes the stream
     h->has_terrain = false;
     h->seeded = false;
+    h->front = false;
     h->steps = 0;
     h->stop = VCA_STOP_RUNNING;
     return VCA_OK;
@@ -2424,7 +2282,8 @@ vca_status vca_ca_apply_terrain(vca_ca* h, const int32_t* heights) {
     }
     VCA_CUDA(cudaMemcpyAsync(h->heights_dev, hv.data(), sizeof(int32_t) * cols, cudaMemcpyHostToDevice, h->stream));
     VCA_CUDA(cudaMemcpyAsync(h->spill, spill.data(), sizeof(int32_t) * cols, cudaMemcpyHostToDevice, h->stream));
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
+    h->front_listed = false;
     ca_terrain_kernel<<<1184, 256, 0, h->stream>>>(h->type[cur], h->heights_dev, g.nx, g.ny, g.nz, g.P);
     VCA_CUDA(cudaGetLastError());
     VCA_CUDA(cudaStreamSynchronize(h->stream));
@@ -2442,7 +2301,7 @@ vca_status vca_ca_place_seeds(vca_ca* h, const vca_vent* vents, int count) {
     }
     VCA_CUDA(cudaSetDevice(h->device));
     const auto& g = h->geom;
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
     const float temp = h->desc.mode == VCA_MODE_LAVA ? h->desc.erupt_temp : 0.0f;
     std::vector<int4> seeds((size_t)count);
     for (int i = 0; i < count; ++i) {
@@ -2503,6 +2362,8 @@ vca_status vca_ca_set_state(vca_ca* h, const uint8_t* type, const int32_t* flow_
     VCA_CUDA(cudaSetDevice(h->device));
     const auto& g = h->geom;
     const int cur = steps_done & 1;
+    h->front = false;
+    h->steps = steps_done;
     if (vca_status s = put_plane(h, h->type[cur], type)) return s;
     if (vca_status s = put_plane(h, h->flow[cur], flow_id)) return s;
     if (vca_status s = put_plane(h, h->temp[cur], temp)) return s;
@@ -2552,8 +2413,9 @@ vca_status vca_ca_get_info(vca_ca* h, vca_ca_info* out) {
     out->lava_cells = h->ctrl_host->lava;
     out->air_cells = h->ctrl_host->air;
     out->tiles_total = h->ntiles;
-    out->tiles_processed = h->ctrl_host->tiles_processed;
     out->cells_per_tile = (uint64_t)kTileX * h->geom.TY * h->geom.TZ;
+    out->tiles_processed = h->ctrl_host->tiles_processed;
+    if (h->front) out->tiles_processed = (out->tiles_processed + out->cells_per_tile - 1) / out->cells_per_tile;
     out->kernel_launches = h->launches;
     return VCA_OK;
 }
@@ -2577,7 +2439,7 @@ vca_status vca_ca_download(vca_ca* h, uint8_t* type, int32_t* flow_id, float* te
     if (vca_status s = not_in_batch(h, "vca_ca_download")) return s;
     VCA_CUDA(cudaSetDevice(h->device));
     if (vca_status s = sync_ctrl(h)) return s;
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
     if (type) if (vca_status s = get_plane(h, type, h->type[cur])) return s;
     if (flow_id) if (vca_status s = get_plane(h, flow_id, h->flow[cur])) return s;
     if (temp) if (vca_status s = get_plane(h, temp, h->temp[cur])) return s;
@@ -2618,7 +2480,7 @@ vca_status vca_ca_flow_stats(vca_ca* h, int flows, uint64_t* lava, uint64_t* bas
         h->flow_sums_cap = 3 * m;
     }
     VCA_CUDA(cudaMemsetAsync(h->flow_sums, 0, sizeof(unsigned long long) * 3 * m, h->stream));
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
     const auto& g = h->geom;
     const size_t smem = flows <= kFlowPrivMax ? sizeof(unsigned long long) * 3 * m : 0;
     const uint64_t cells = (uint64_t)g.nx * g.ny * g.nz;
@@ -2701,7 +2563,7 @@ vca_status vca_ca_layers(vca_ca* h, void** type, void** flow_id, void** temp, vo
     if (vca_status s = not_in_batch(h, "vca_ca_layers")) return s;
     VCA_CUDA(cudaSetDevice(h->device));
     if (vca_status s = sync_ctrl(h)) return s;
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
     if (type) *type = h->type[cur];
     if (flow_id) *flow_id = h->flow[cur];
     if (temp) *temp = h->temp[cur];
@@ -2727,7 +2589,8 @@ static vca_status layers_check(vca_ca* h, int z0, int types, int full, const voi
 static vca_status copy_layers(vca_ca* h, int z0, int types, int full, void* buf, bool to_buf) {
     VCA_CUDA(cudaSetDevice(h->device));
     if (vca_status s = sync_ctrl(h)) return s;
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
+    if (!to_buf) h->front_listed = false;  // the copied layers may hold other LAVA cells
     const size_t L = (size_t)h->geom.P * h->geom.ny;
     char* b = static_cast<char*>(buf);
     auto move = [&](void* plane, size_t elem, int z, int n, size_t at) -> cudaError_t {
@@ -2791,7 +2654,7 @@ vca_status ca_view(vca_ca* h, CaView* v) {
     if (vca_status s = check(h)) return s;
     if (vca_status s = not_in_batch(h, "vca_mc_set_domain_from_ca / vca_mc_set_mobility_from_ca")) return s;
     if (vca_status s = sync_ctrl(h)) return s;
-    const int cur = h->steps & 1;
+    const int cur = h->cur();
     v->type = h->type[cur];
     v->solid = h->solid[cur];
     v->arrival = h->arrival[cur];
@@ -2811,7 +2674,8 @@ vca_status ca_view(vca_ca* h, CaView* v) {
 struct vca_ca_batch {
     int device = 0;
     int cap = 0;                  // member slots
-    int rules_grid = 0, cand_grid = 0;
+    int rules_grid = 0, cand_grid = 0, front_grid = 0;
+    int tile_members = 0, front_members = 0;  // as of the tables on the device
     cudaStream_t stream = nullptr;
     // device tables
     CaTensorMaps* d_tm = nullptr;
@@ -2820,9 +2684,13 @@ struct vca_ca_batch {
     int2* d_cand_map = nullptr;
     int* d_rules_n = nullptr;
     int* d_cand_n = nullptr;
-    int4* d_status = nullptr;
-    int4* h_status = nullptr;     // pinned, two ring slots of cap entries: (stop, error, steps, next tiles)
-    std::vector<uint64_t> weight; // per slot: tiles of the member's next step (its share of the blocks)
+    CaFrontArgs* d_front_args = nullptr;
+    int2* d_front_map = nullptr;
+    int* d_front_n = nullptr;
+    CaCtrl** d_ctrl = nullptr;    // per slot: the member's control block
+    int4* h_status = nullptr;     // pinned, host-mapped: two ring slots of cap entries (stop, error, steps, next size)
+    int4* h_status_dev = nullptr; // its device address
+    std::vector<uint64_t> weight; // per slot: the size of the member's next step, tiles or front cells
     cudaEvent_t status_ev[2] = {nullptr, nullptr};
     cudaEvent_t sync_ev = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -2831,6 +2699,7 @@ struct vca_ca_batch {
     std::vector<vca_ca*> early;   // members that had stopped before they were added
     std::vector<vca_ca*> done;    // stopped members not yet handed out
     bool dirty = true;            // tables on the device are out of date
+    bool resplit = false;         // only the split of the blocks is
     int pending = -1;             // ring slot whose status is not read yet
     int ring = 0;
     uint64_t graphs = 0, launches = 0;
@@ -2881,45 +2750,71 @@ void split_blocks(const std::vector<uint64_t>& w, int grid, std::vector<int>& n)
     }
 }
 
-// Member arguments and block maps to the device (on the batch stream, ordered after the graphs
-// already launched and before the next).
+// Blocks of the front launch that a list of n cells can use: a block per 256 cells.
+int front_share(uint64_t n) { return (int)std::min<uint64_t>(n / kFrontBatchThreads + 1, 1u << 20); }
+
+// Block maps (and, when the members changed, their arguments) to the device, on the batch stream,
+// ordered after the launches already queued and before the next.
 vca_status batch_upload(vca_ca_batch* b) {
-    std::vector<CaTensorMaps> tm((size_t)b->cap);
-    std::vector<CaKernelArgs> args((size_t)b->cap);
-    std::vector<int> rn((size_t)b->cap, 0), cn((size_t)b->cap, 0);
+    const size_t cap = (size_t)b->cap;
+    std::vector<int> rn(cap, 0), cn(cap, 0), fn(cap, 0);
     std::vector<int2> rmap((size_t)b->rules_grid, make_int2(-1, 0)), cmap((size_t)b->cand_grid, make_int2(-1, 0));
-    std::vector<int> members;
-    std::vector<uint64_t> w;
+    std::vector<int2> fmap((size_t)b->front_grid, make_int2(-1, 0));
+    std::vector<int> tile, front;
+    std::vector<uint64_t> tile_w, front_w;
     for (int i = 0; i < b->cap; ++i) {
         vca_ca* h = b->slots[(size_t)i];
-        std::memset(&args[(size_t)i], 0, sizeof(CaKernelArgs));
         if (!h) continue;
-        tm[(size_t)i] = h->tmaps;
-        args[(size_t)i] = make_args(h, true);
-        members.push_back(i);
-        w.push_back(std::max<uint64_t>(1, b->weight[(size_t)i]));
+        (h->front ? front : tile).push_back(i);
+        (h->front ? front_w : tile_w).push_back(std::max<uint64_t>(1, b->weight[(size_t)i]));
     }
-    std::vector<int> nr, nc;
-    split_blocks(w, b->rules_grid, nr);
-    split_blocks(w, b->cand_grid, nc);
-    int at_r = 0, at_c = 0;
-    for (size_t j = 0; j < members.size(); ++j) {
-        const int slot = members[j];
-        rn[(size_t)slot] = nr[j];
-        cn[(size_t)slot] = nc[j];
-        for (int q = 0; q < nr[j]; ++q) rmap[(size_t)(at_r + q)] = make_int2(slot, q);
-        for (int q = 0; q < nc[j]; ++q) cmap[(size_t)(at_c + q)] = make_int2(slot, q);
-        at_r += nr[j];
-        at_c += nc[j];
-    }
+    auto share = [](const std::vector<int>& members, const std::vector<int>& n, std::vector<int>& per_slot, std::vector<int2>& map) {
+        int at = 0;
+        for (size_t j = 0; j < members.size(); ++j) {
+            per_slot[(size_t)members[j]] = n[j];
+            for (int q = 0; q < n[j]; ++q) map[(size_t)at++] = make_int2(members[j], q);
+        }
+    };
+    std::vector<int> nr, nc, nf;
+    split_blocks(tile_w, b->rules_grid, nr);
+    split_blocks(tile_w, b->cand_grid, nc);
+    split_blocks(front_w, b->front_grid, nf);
+    for (size_t j = 0; j < front.size(); ++j) nf[j] = std::min(nf[j], front_share(front_w[j] + front_w[j] / 4));
+    share(tile, nr, rn, rmap);
+    share(tile, nc, cn, cmap);
+    share(front, nf, fn, fmap);
+    b->tile_members = (int)tile.size();
+    b->front_members = (int)front.size();
     // pageable sources: each copy is staged before the call returns, so the vectors may go
-    VCA_CUDA(cudaMemcpyAsync(b->d_tm, tm.data(), sizeof(CaTensorMaps) * tm.size(), cudaMemcpyHostToDevice, b->stream));
-    VCA_CUDA(cudaMemcpyAsync(b->d_args, args.data(), sizeof(CaKernelArgs) * args.size(), cudaMemcpyHostToDevice, b->stream));
-    VCA_CUDA(cudaMemcpyAsync(b->d_rules_n, rn.data(), sizeof(int) * rn.size(), cudaMemcpyHostToDevice, b->stream));
-    VCA_CUDA(cudaMemcpyAsync(b->d_cand_n, cn.data(), sizeof(int) * cn.size(), cudaMemcpyHostToDevice, b->stream));
-    VCA_CUDA(cudaMemcpyAsync(b->d_rules_map, rmap.data(), sizeof(int2) * rmap.size(), cudaMemcpyHostToDevice, b->stream));
-    VCA_CUDA(cudaMemcpyAsync(b->d_cand_map, cmap.data(), sizeof(int2) * cmap.size(), cudaMemcpyHostToDevice, b->stream));
-    b->dirty = false;
+    auto put = [&](void* to, const void* from, size_t bytes) { return cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, b->stream); };
+    VCA_CUDA(put(b->d_front_n, fn.data(), sizeof(int) * cap));
+    VCA_CUDA(put(b->d_front_map, fmap.data(), sizeof(int2) * fmap.size()));
+    if (!tile.empty() || b->dirty) {
+        VCA_CUDA(put(b->d_rules_n, rn.data(), sizeof(int) * cap));
+        VCA_CUDA(put(b->d_cand_n, cn.data(), sizeof(int) * cap));
+        VCA_CUDA(put(b->d_rules_map, rmap.data(), sizeof(int2) * rmap.size()));
+        VCA_CUDA(put(b->d_cand_map, cmap.data(), sizeof(int2) * cmap.size()));
+    }
+    if (b->dirty) {
+        std::vector<CaCtrl*> ctrl(cap, nullptr);
+        std::vector<CaFrontArgs> fargs(cap);
+        for (int i : front) fargs[(size_t)i] = front_args(b->slots[(size_t)i]);
+        for (int i = 0; i < b->cap; ++i)
+            if (b->slots[(size_t)i]) ctrl[(size_t)i] = b->slots[(size_t)i]->ctrl;
+        VCA_CUDA(put(b->d_ctrl, ctrl.data(), sizeof(CaCtrl*) * cap));
+        if (!front.empty()) VCA_CUDA(put(b->d_front_args, fargs.data(), sizeof(CaFrontArgs) * cap));
+        if (!tile.empty()) {
+            std::vector<CaTensorMaps> tm(cap);
+            std::vector<CaKernelArgs> args(cap);
+            for (int i : tile) {
+                tm[(size_t)i] = b->slots[(size_t)i]->tmaps;
+                args[(size_t)i] = make_args(b->slots[(size_t)i]);
+            }
+            VCA_CUDA(put(b->d_tm, tm.data(), sizeof(CaTensorMaps) * cap));
+            VCA_CUDA(put(b->d_args, args.data(), sizeof(CaKernelArgs) * cap));
+        }
+    }
+    b->dirty = b->resplit = false;
     return VCA_OK;
 }
 
@@ -2952,26 +2847,28 @@ vca_status batch_collect(vca_ca_batch* b, int r) {
             b->done.push_back(h);
             continue;
         }
-        // the blocks follow the work: re-split when a member's visited tiles moved by more than 1/8
-        const uint64_t now = std::max<uint64_t>(1, (uint64_t)std::max(0, st[i].w));
+        // the blocks follow the work: re-split when a member's visited tiles moved by more than 1/8, or
+        // the blocks its front list can use by more than a quarter
+        const uint64_t now = std::max<uint64_t>(1, (uint64_t)(uint32_t)st[i].w);
         uint64_t& was = b->weight[(size_t)i];
-        if (now > was + was / 8 || now + now / 8 < was) {
+        const bool moved = h->front ? front_share(now) > front_share(was + was / 4) || 2 * now < was
+                                    : now > was + was / 8 || now + now / 8 < was;
+        if (moved) {
             was = now;
-            b->dirty = true;
+            b->resplit = true;
         }
     }
     return VCA_OK;
 }
 
 vca_status batch_capture(vca_ca_batch* b) {
-    CaBatchView v{b->d_tm, b->d_args, b->d_rules_map, b->d_cand_map, b->d_rules_n, b->d_cand_n, b->d_status, b->cap};
+    CaBatchView v{b->d_tm, b->d_args, b->d_rules_map, b->d_cand_map, b->d_rules_n, b->d_cand_n};
     VCA_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     for (int s = 0; s < kGraphSteps; ++s) {
         ca_drop_batch_kernel<<<b->rules_grid, kThreads, 0, b->stream>>>(v);
         ca_rules_batch_kernel<<<b->rules_grid, kThreads, kRulesDynSmem, b->stream>>>(v);
         ca_cand_batch_kernel<<<b->cand_grid, kCandThreads, 0, b->stream>>>(v);
     }
-    ca_batch_status_kernel<<<1, 256, 0, b->stream>>>(v);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
@@ -2993,7 +2890,10 @@ void batch_free(vca_ca_batch* b) {
     cudaFree(b->d_cand_map);
     cudaFree(b->d_rules_n);
     cudaFree(b->d_cand_n);
-    cudaFree(b->d_status);
+    cudaFree(b->d_front_args);
+    cudaFree(b->d_front_map);
+    cudaFree(b->d_front_n);
+    cudaFree(b->d_ctrl);
     if (b->h_status) cudaFreeHost(b->h_status);
     for (cudaEvent_t e : b->status_ev)
         if (e) cudaEventDestroy(e);
@@ -3037,7 +2937,12 @@ vca_status vca_ca_batch_create(int device, int max_members, vca_ca_batch** out) 
         return fail(cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor"));
     b->rules_grid = prop.multiProcessorCount * std::max(1, rules_per_sm);
     b->cand_grid = prop.multiProcessorCount * std::max(1, cand_per_sm);
-    b->cap = std::min(max_members, std::min(b->rules_grid, b->cand_grid));
+    b->front_grid = front_batch_grid(prop.multiProcessorCount);
+    b->cap = std::min(max_members, std::min(b->rules_grid, std::min(b->cand_grid, b->front_grid)));
+    if (b->cap < 1) {
+        set_error("vca_ca_batch_create: the batched kernels do not fit this device");
+        return fail(VCA_ERR_CUDA);
+    }
     b->slots.assign((size_t)b->cap, nullptr);
     b->weight.assign((size_t)b->cap, 1);
     if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess)
@@ -3053,10 +2958,14 @@ vca_status vca_ca_batch_create(int device, int max_members, vca_ca_batch** out) 
     BALLOC(b->d_cand_map, sizeof(int2) * (size_t)b->cand_grid);
     BALLOC(b->d_rules_n, sizeof(int) * (size_t)b->cap);
     BALLOC(b->d_cand_n, sizeof(int) * (size_t)b->cap);
-    BALLOC(b->d_status, sizeof(int4) * (size_t)b->cap);
+    BALLOC(b->d_front_args, sizeof(CaFrontArgs) * (size_t)b->cap);
+    BALLOC(b->d_front_map, sizeof(int2) * (size_t)b->front_grid);
+    BALLOC(b->d_front_n, sizeof(int) * (size_t)b->cap);
+    BALLOC(b->d_ctrl, sizeof(CaCtrl*) * (size_t)b->cap);
 #undef BALLOC
-    if ((e = cudaMallocHost(&b->h_status, sizeof(int4) * 2 * (size_t)b->cap)) != cudaSuccess)
-        return fail(cuda_fail(e, "cudaMallocHost"));
+    if ((e = cudaHostAlloc(&b->h_status, sizeof(int4) * 2 * (size_t)b->cap, cudaHostAllocMapped)) != cudaSuccess ||
+        (e = cudaHostGetDevicePointer(&b->h_status_dev, b->h_status, 0)) != cudaSuccess)
+        return fail(cuda_fail(e, "cudaHostAlloc (mapped)"));
     if ((e = cudaEventCreateWithFlags(&b->status_ev[0], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->status_ev[1], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->sync_ev, cudaEventDisableTiming)) != cudaSuccess)
@@ -3101,11 +3010,13 @@ vca_status vca_ca_batch_add(vca_ca_batch* b, vca_ca* h) {
         set_error("vca_ca_batch_add: the batch is full (" + std::to_string(b->cap) + " members)");
         return VCA_ERR_ARG;
     }
+    if (h->front && !h->front_listed)
+        if (vca_status s = front_list(h)) return s;
     // the batch's next launches come after the member's set-up work
     VCA_CUDA(cudaEventRecord(b->sync_ev, h->stream));
     VCA_CUDA(cudaStreamWaitEvent(b->stream, b->sync_ev, 0));
     b->slots[(size_t)slot] = h;
-    b->weight[(size_t)slot] = std::max<uint64_t>(1, h->ntiles);  // until its first status
+    b->weight[(size_t)slot] = std::max<uint64_t>(1, h->front ? h->ctrl_host->front_n : h->ntiles);  // until its first status
     h->batch = b;
     h->batch_slot = slot;
     b->dirty = true;
@@ -3132,16 +3043,25 @@ vca_status vca_ca_batch_advance(vca_ca_batch* b, int max_graphs, vca_ca** finish
     };
     for (int g = 0; g < max_graphs && b->done.empty(); ++g) {
         if (members() == 0) break;
-        if (b->dirty)
+        if (b->dirty || b->resplit)
             if (vca_status s = batch_upload(b)) return s;
         const int r = b->ring;
-        VCA_CUDA(cudaGraphLaunch(b->graph, b->stream));
-        VCA_CUDA(cudaMemcpyAsync(b->h_status + (size_t)r * b->cap, b->d_status, sizeof(int4) * (size_t)b->cap,
-                                 cudaMemcpyDeviceToHost, b->stream));
+        if (b->tile_members) {
+            VCA_CUDA(cudaGraphLaunch(b->graph, b->stream));
+            b->launches += 3 * kGraphSteps;
+        }
+        if (b->front_members) {
+            VCA_CUDA(front_batch_launch(CaFrontBatch{b->d_front_args, b->d_front_map, b->d_front_n}, b->front_grid, kGraphSteps,
+                                        b->stream));
+            b->launches += 1;
+        }
+        ca_batch_status_kernel<<<1, 256, 0, b->stream>>>(b->d_ctrl, b->d_front_n,
+                                                         reinterpret_cast<volatile int*>(b->h_status_dev + (size_t)r * b->cap), b->cap);
+        VCA_CUDA(cudaGetLastError());
         VCA_CUDA(cudaEventRecord(b->status_ev[r], b->stream));
         b->snap[r] = b->slots;
         b->graphs += 1;
-        b->launches += 3 * kGraphSteps + 1;
+        b->launches += 1;
         b->ring ^= 1;
         if (b->pending >= 0) {
             if (vca_status s = batch_collect(b, b->pending)) return s;

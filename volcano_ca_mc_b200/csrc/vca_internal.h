@@ -46,6 +46,15 @@ struct CaCtrl {
     int32_t classic;
     int32_t error;            // bit 0: a bounded device wait ran out (the run stops, VCA_ERR_TIMEOUT)
     uint32_t tile_next;       // rules pass (DENSE): tiles handed out at run time in the running step
+    // front kernels (front.cu)
+    uint32_t front_n;         // slots of the front list
+    uint32_t front_prev;      // its slots when the last step began: the later ones were born in that step
+    uint32_t front_exit;      // blocks that have left the running launch
+    uint32_t front_pad;
+    // step t at [t % 3]: the barrier words after its two phases, and the candidates and solidifying
+    // slots that did not fit their block's shared lists
+    unsigned long long front_word[3][2];
+    uint32_t front_over[3][2];
 };
 
 // Geometry of the pitched device planes.  Each (y, z) row holds P >= nx cells, P a multiple of 64,
@@ -119,6 +128,48 @@ struct CaKernelArgs {
     uint64_t gidx_base;
     int own_z0, own_z1;
     int slab;
+};
+
+// The front form of a step (front.cu): the state planes in place, and the list of LAVA cells.
+struct CaFrontArgs {
+    CaGeom g;
+    FastDiv32 div_nx, div_ny;
+    int classic, ponding, diag_falls, random_nb;
+    uint32_t side_mask;       // side offsets (dz = 0) as bits 3 (dy + 1) + (dx + 1)
+    uint32_t vmask[6];        // per variant: bit (dx + 1) + 3 (dy + 1) + 9 (dz + 1) of each offset
+    uint32_t umask;           // their union
+    int max_steps, eruption_steps;
+    float erupt_temp, solidus, cool_ambient, cool_lateral, cool_fall;
+    uint64_t seed;
+    FastMod var_mod;
+    int variants;
+    uint8_t* type;
+    int32_t* flow;
+    float* temp;              // of LAVA cells: written back from the list at the end of a launch
+    uint16_t* solid;
+    uint16_t* arrival;
+    const int32_t* spill;     // nx*ny or nullptr
+    const int4* vents;
+    int vent_slots;
+    uint32_t* mark;           // per cell: the sources that reach it in this step (0 between steps)
+    uint32_t* stamp;          // per column: the last step that changed a type in it or beside it
+    uint32_t* idx;            // per slot: globalIndex
+    float* ltemp;             // per slot: temperature
+    uint8_t* flags;           // per slot: kFront*
+    uint32_t* work;           // overflow lists: candidates from the bottom, solidifying slots from the top
+    uint32_t work_cap;
+    uint32_t pad;
+    CaCtrl* ctrl;
+    unsigned long long* hist_active;
+    unsigned long long* hist_changed;
+};
+
+// A batched front launch: per member slot its arguments and blocks, per block its member and index.
+constexpr int kFrontBatchThreads = 256;
+struct CaFrontBatch {
+    const CaFrontArgs* args;
+    const int2* map;          // (member slot or -1, block within the member)
+    const int* n;             // blocks of each slot
 };
 
 // Read-only view of a CA handle's current planes (the MC domain and mobility are built from it).
@@ -212,4 +263,22 @@ struct vca_ca {
     // z slab of a taller grid (vca_ca_set_slab); slab_z0 = global z of local layer 0
     bool slab = false;
     int slab_z0 = 0, own_z0 = 0, own_z1 = 0;
+    // stepped by the front kernels: the state stays in buffer front_buf (the other buffer is their
+    // scratch); front_listed = the front list matches the planes
+    bool front = false;
+    int front_buf = 0;
+    bool front_listed = false;
+    // the buffer that holds the current state
+    int cur() const { return front ? front_buf : steps & 1; }
 };
+
+namespace vca {
+// front.cu: the front form of the ACTIVE schedule
+CaFrontArgs front_args(const vca_ca* h);
+vca_status front_init(vca_ca* h, int steps_done);                   // marks cleared, list and totals from the planes
+vca_status front_list(vca_ca* h);                                   // the same, the totals kept
+vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop);
+int front_batch_grid(int sms);                                      // blocks of a batched launch, 0 on failure
+cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cudaStream_t stream);
+vca_status sync_ctrl(vca_ca* h);
+}  // namespace vca

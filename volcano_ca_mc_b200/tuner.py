@@ -9,7 +9,7 @@ counterpart: its nearest knob is the OpenMP schedule and chunk of the CPU sweep
 
 A shape class is (dimensionality, neighbourhood, log2 of the cell count).  For each class the tuner
 times every candidate launch shape on a calibration job -- a seeded Gaussian-cone terrain of the
-class's size with a few vents, run for a fixed number of ACTIVE steps from the same start -- and
+class's size with a few vents, run for a fixed number of tile-list (ACTIVE_LIST) steps from the same start -- and
 keeps the fastest.  Cells per thread are fixed at 4 (one 32-bit byte window per thread in the rules
 pass), so they are not a tuned knob.
 
@@ -75,12 +75,12 @@ def calibration_terrain(nx: int, ny: int, nz: int, seed: int = 11):
 
 
 def time_candidate(nx, ny, nz, neighborhood, cand, steps, heights, vents, device=0, reps=2) -> float:
-    """Device time [ms] of `steps` ACTIVE steps of the calibration job with this launch shape (the best
+    """Device time [ms] of `steps` tile-list steps of the calibration job with this launch shape (the best
     of `reps` runs on one handle)."""
     ty, tz, b = cand
     p = capi.CaParams(nx, ny, nz, neighborhood=neighborhood, boundary="absorbing", seed=5, max_steps=steps,
                       eruption_steps=steps, cooling_ambient=2.0, cooling_lateral=4.0, cooling_fall=2.0, device=device,
-                      tile_y=ty, tile_z=tz, rules_blocks_per_sm=b)
+                      tile_y=ty, tile_z=tz, rules_blocks_per_sm=b, sweep=capi.SWEEP_ACTIVE_LIST)
     ca = capi.LavaCA(p)
     best = float("inf")
     for r in range(reps + 1):
@@ -194,7 +194,7 @@ def main():
         table["classes"][cls] = tune_class(cls, args.steps)
         print(cls, table["classes"][cls]["tile"], table["classes"][cls]["rules_blocks_per_sm"],
               table["classes"][cls]["ms"], flush=True)
-    table["note"] = ("launch shape per class: the fastest on the calibration job's ACTIVE steps unless the default "
+    table["note"] = ("launch shape per class: the fastest on the calibration job's tile-list steps unless the default "
                      "4x4/b0 is within 3 % of it (tuner.tune_class); results are identical for every shape")
     with open(args.out, "w") as f:
         json.dump(table, f, indent=1)
