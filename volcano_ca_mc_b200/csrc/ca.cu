@@ -1369,19 +1369,6 @@ __global__ void ca_pad_kernel(uint8_t* t0, uint8_t* t1, int nx, int P, int64_t r
     }
 }
 
-// ROCK for z < h(x, y) (LavaCA::applyTerrain, LavaCA.hpp:185-194).
-__global__ void ca_terrain_kernel(uint8_t* type, const int32_t* heights, int nx, int ny, int nz, int P) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const int64_t r = i / nx;
-        const int y = (int)(r % ny);
-        const int z = (int)(r / ny);
-        const int h = min(heights[x + (int64_t)nx * y], nz);
-        if (z < h) type[x + (int64_t)P * r] = kRock;
-    }
-}
-
 // ------------------------------------------------------------------------------------------
 // Batched stepping: one launch of each step kernel for many grids.  Every block serves one member
 // grid: the block maps give, per block of a launch, the member slot and the block's index among that
@@ -2266,29 +2253,15 @@ vca_status vca_ca_apply_terrain(vca_ca* h, const int32_t* heights) {
     VCA_CUDA(cudaSetDevice(h->device));
     const auto& g = h->geom;
     const size_t cols = (size_t)g.nx * g.ny;
-    std::vector<int32_t> hv(heights, heights + cols);
-    for (auto& v : hv) {
-        if (v < 0) {
-            set_error("vca_ca_apply_terrain: negative height");
-            return VCA_ERR_ARG;
-        }
+    int32_t lowest = heights[0];
+    for (size_t i = 1; i < cols; ++i) lowest = std::min(lowest, heights[i]);
+    if (lowest < 0) {
+        set_error("vca_ca_apply_terrain: negative height");
+        return VCA_ERR_ARG;
     }
-    std::vector<int32_t> spill = fill_depressions(hv, g.nx, g.ny, g.per[0] != 0, g.per[1] != 0);
-    if (h->slab) {
-        // heights and spill levels of the whole grid, seen from this slab's layer 0: every test
-        // against them (z < h, z - 1 < spill, z <= spill) keeps its truth with both sides shifted
-        for (auto& v : hv) v -= h->slab_z0;
-        for (auto& v : spill) v -= h->slab_z0;
-    }
-    VCA_CUDA(cudaMemcpyAsync(h->heights_dev, hv.data(), sizeof(int32_t) * cols, cudaMemcpyHostToDevice, h->stream));
-    VCA_CUDA(cudaMemcpyAsync(h->spill, spill.data(), sizeof(int32_t) * cols, cudaMemcpyHostToDevice, h->stream));
-    const int cur = h->cur();
     h->front_listed = false;
-    ca_terrain_kernel<<<1184, 256, 0, h->stream>>>(h->type[cur], h->heights_dev, g.nx, g.ny, g.nz, g.P);
-    VCA_CUDA(cudaGetLastError());
-    VCA_CUDA(cudaStreamSynchronize(h->stream));
+    if (vca_status s = terrain_apply(h, heights, lowest)) return s;
     h->has_terrain = true;
-    h->launches += 1;
     return VCA_OK;
 }
 

@@ -281,4 +281,6 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop);
 int front_batch_grid(int sms);                                      // blocks of a batched launch, 0 on failure
 cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cudaStream_t stream);
 vca_status sync_ctrl(vca_ca* h);
+// terrain.cu: heights and spill levels into their planes, ROCK columns
+vca_status terrain_apply(vca_ca* h, const int32_t* heights, int32_t lowest);
 }  // namespace vca
