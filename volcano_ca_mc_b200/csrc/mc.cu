@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "vca.h"
@@ -532,17 +533,35 @@ __global__ __launch_bounds__(kMcThreads, 2) void mc_sweeps_kernel(const __grid_c
 
 // ------------------------------------------------------------------------------------------
 // Whole-space domain (mc.domain = full, every cell a trial each MCS) with Q <= 256: the sweeps run on
-// a one-byte copy of the orientations (orientation - 1, so 67 M cells take 67 MB and stay in L2) and
-// enumerate the cells of each colour class directly instead of reading a list.  A cell's neighbours
-// are loaded at fixed linear offsets when the cell is away from every face (no wrap or frame test),
-// else through the frame as everywhere else.  Same trials, same order of colours, same results.
+// a one-byte copy of the orientations (orientation - 1, so 67 M cells take 69 MB and stay in L2).
+//
+// A thread takes the four cells of a colour among eight neighbouring x (every colour steps by two in x)
+// and counts their unlike neighbours four bytes at a time: per row of the 3 x 3 x 3 block one aligned
+// 8-byte load and one byte beside it give the left, middle and right neighbours of the four cells as
+// three words; a byte of x = word ^ orientations is zero where the neighbour is alike, and x + 0x7f..
+// has bit 7 set where it is not (Q <= 128).  The 26 words are added as one-bit numbers with bitwise
+// adders, about half the operations of shifting each into a byte counter.
+//
+// The copy has rows of P8 bytes: 8 in front (the last one holds the orientation at x = nx - 1, the left
+// neighbour of x = 0 on a wrapped axis), nx cells, the orientation at x = 0, and room for the last load.
+// What bounds it: the integer ALU (79 % busy), three 64-bit hashes of a trial (two at kT = 0) above all.
+// Per MCS on one B200 against a thread per cell with 26 byte loads and compares (709 instructions per
+// trial): 512 x 512 x 256 Moore, Q = 64, kT = 0.5 1.80 -> 0.79 ms, the same von Neumann 1.88 -> 0.54 ms,
+// 256 x 256 x 128 pentagonal 0.30 -> 0.16 ms, 50^3 Moore 38 -> 29 us.  Three resident blocks per SM
+// instead of two (80 registers, spills) 0.85 ms; moving adds and shifts to the FMA pipe 0.89 ms.
 // ------------------------------------------------------------------------------------------
-struct McDense {
-    uint8_t* sp;             // orientation - 1 of every cell
+constexpr int kSpaceBlocks = 2;  // resident blocks per SM the registers are limited to
+struct McSpace {
+    uint8_t* sp;             // P8-byte rows: orientation - 1
     const float* mob;        // mobility of every cell (kMobility)
-    int cnt[3][3];           // per axis and class: coordinates of the class
-    FastDiv32 div[2][3];     // / cnt[0][c] and / cnt[1][c]
+    int P8;
+    int gx[3], g0[3];        // groups of 8 x per row that hold cells of x class c, the first one
+    int xlo[3], xhi[3];      // x range of class c (its parity: c & 1)
+    int cnt[3][3];           // per axis and class: coordinates of the class (y and z)
+    FastDiv32 div_gx[3], div_cy[3];
+    uint32_t qm1, qm1_inv, qm1_2p32;  // Q - 1, floor((2^32 - 1) / (Q - 1)), 2^32 mod (Q - 1)
     uint32_t mask[6];        // per variant: bit (dx + 1) + 3 (dy + 1) + 9 (dz + 1) of each neighbour
+    int uphill;              // kT > 0: some uphill moves are accepted
 };
 
 // Coordinate i of class c on an axis of n cells split into `classes` classes (axisClass,
@@ -552,95 +571,347 @@ __device__ __forceinline__ int class_coord(int i, int c, int classes, int n) {
     return classes == 1 ? i : (c == 2 ? n - 1 : 2 * i + c);
 }
 
-__global__ void mc_pack8_kernel(const int32_t* spin, uint8_t* sp, uint64_t n) {
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x)
-        sp[g] = (uint8_t)(spin[g] - 1);
+// The byte copy of the orientations with its frame columns, and back.  A thread moves the cells of one
+// group of eight.
+__global__ void mc_pack8_kernel(const int32_t* spin, uint8_t* sp, int nx, int P8, uint64_t rows) {
+    const int groups = P8 / 8 - 2;
+    const uint64_t n = (uint64_t)groups * rows;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t row = i / (uint64_t)groups;
+        const int x0 = 8 * (int)(i - row * (uint64_t)groups);
+        const int32_t* from = spin + row * (uint64_t)nx;
+        uint8_t* to = sp + row * (uint64_t)P8 + 8;
+        uint32_t w[2] = {0, 0};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int x = x0 + j;
+            // past the row: x = nx is the frame column
+            const int32_t v = x < nx ? from[x] : from[0];
+            w[j >> 2] |= (uint32_t)(uint8_t)(v - 1) << (8 * (j & 3));
+        }
+        *reinterpret_cast<uint2*>(to + x0) = make_uint2(w[0], w[1]);
+        if (x0 == 0) to[-1] = (uint8_t)(from[nx - 1] - 1);
+        if (x0 + 8 == nx) to[nx] = (uint8_t)(from[0] - 1);
+    }
 }
-__global__ void mc_unpack8_kernel(const uint8_t* sp, int32_t* spin, uint64_t n) {
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x)
-        spin[g] = (int32_t)sp[g] + 1;
+__global__ void mc_unpack8_kernel(const uint8_t* sp, int32_t* spin, int nx, int P8, uint64_t rows) {
+    const int groups = P8 / 8 - 2;
+    const uint64_t n = (uint64_t)groups * rows;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t row = i / (uint64_t)groups;
+        const int x0 = 8 * (int)(i - row * (uint64_t)groups);
+        const uint2 v = *reinterpret_cast<const uint2*>(sp + row * (uint64_t)P8 + 8 + x0);
+        int32_t* to = spin + row * (uint64_t)nx + x0;
+        int32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = (int32_t)(((j < 4 ? v.x : v.y) >> (8 * (j & 3))) & 0xFFu) + 1;
+        if ((nx & 3) == 0 && x0 + 8 <= nx) {
+            *reinterpret_cast<int4*>(to) = make_int4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<int4*>(to + 4) = make_int4(o[4], o[5], o[6], o[7]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (x0 + j < nx) to[j] = o[j];
+        }
+    }
 }
 
-// kMoore3: the 26-cell Moore neighbourhood of a 3D space, whose interior cells read their 26
-// neighbours from nine row addresses and immediate offsets.
-template <bool kMobility, bool kRandomNb, bool kParity, bool kMoore3>
-__global__ __launch_bounds__(kMcThreads, 3) void mc_dense_sweeps_kernel(const __grid_constant__ McArgs a,
-                                                                        const __grid_constant__ McDense d, int sweeps) {
+// x mod d for d <= 255 from the 32-bit halves: hi (2^32 mod d) + lo, each remainder below 2 d (the
+// quotient is exact or one too small), is below 2^18; the last remainder is finished by one subtraction.
+__device__ __forceinline__ uint32_t mod_q(const McSpace& d, uint64_t x) {
+    auto rem = [&](uint32_t v) { return v - __umulhi(v, d.qm1_inv) * d.qm1; };
+    const uint32_t r = rem(rem((uint32_t)(x >> 32)) * d.qm1_2p32 + rem((uint32_t)x));
+    return min(r, r - d.qm1);
+}
+
+// Bitwise adders over words of one-bit numbers: sum and carry of three, of two.
+__device__ __forceinline__ void add3(uint32_t a, uint32_t b, uint32_t c, uint32_t& sum, uint32_t& carry) {
+    sum = a ^ b ^ c;
+    carry = (a & b) | (c & (a | b));
+}
+__device__ __forceinline__ void add2(uint32_t a, uint32_t b, uint32_t& sum, uint32_t& carry) {
+    sum = a ^ b;
+    carry = a & b;
+}
+// Numbers of up to four bits, one per byte: bit 7 of each byte of w[i] is bit i (the other bits are unused).
+struct Planes {
+    uint32_t w[4];
+};
+// The nine inputs of a plane of the 3 x 3 x 3 block, given as sum and carry of each row.
+__device__ __forceinline__ Planes add_rows(const uint32_t s[3], const uint32_t c[3]) {
+    Planes p;
+    uint32_t k2, x2, k4, k4b;
+    add3(s[0], s[1], s[2], p.w[0], k2);
+    add3(c[0], c[1], c[2], x2, k4);
+    add2(k2, x2, p.w[1], k4b);
+    add2(k4, k4b, p.w[2], p.w[3]);
+    return p;
+}
+// The sum of three planes (up to 27) as one byte per number.
+__device__ __forceinline__ uint32_t add_planes(const Planes& a, const Planes& b, const Planes& c) {
+    uint32_t p0, p1, p2, p3, p4, c2, x, c4, c4b, y, c8, c8b, z, c16, c16b;
+    add3(a.w[0], b.w[0], c.w[0], p0, c2);
+    add3(a.w[1], b.w[1], c.w[1], x, c4);
+    add2(x, c2, p1, c4b);
+    add3(a.w[2], b.w[2], c.w[2], y, c8);
+    add3(y, c4, c4b, p2, c8b);
+    add3(a.w[3], b.w[3], c.w[3], z, c16);
+    add3(z, c8, c8b, p3, c16b);
+    p4 = c16 | c16b;
+    return ((p0 >> 7) & 0x01010101u) | ((p1 >> 6) & 0x02020202u) | ((p2 >> 5) & 0x04040404u) | ((p3 >> 4) & 0x08080808u) |
+           ((p4 >> 3) & 0x10101010u);
+}
+
+// kNb: 0 the whole 3 x 3 x 3 block (Moore), 1 the six faces (von Neumann), 2 by the variants' masks.
+// kWide: Q > 128, so an orientation - 1 takes all eight bits of its byte.
+template <bool kMobility, int kNb, bool kParity, bool kWide>
+__global__ __launch_bounds__(kMcThreads, kSpaceBlocks) void mc_space_sweeps_kernel(const __grid_constant__ McArgs a,
+                                                                        const __grid_constant__ McSpace d, int sweeps) {
     __shared__ unsigned long long s_table[kTableSide * kTableSide];
     __shared__ unsigned long long s_red[3][kMcThreads / 32];
-    for (int i = threadIdx.x; i < kTableSide * kTableSide; i += kMcThreads) s_table[i] = a.table[i];
+    for (int i = threadIdx.x; i < kTableSide * kTableSide; i += kMcThreads) {
+        // (r >> 11) < th is r < th << 11 as long as that fits
+        const unsigned long long th = a.table[i];
+        s_table[i] = th >> 63 ? 1ull : (th >> 53 ? 2ull : th << 11);
+    }
     __syncthreads();
     McCtrl* ctrl = a.ctrl;
     const uint32_t t0 = ctrl->sweeps;
-    const uint8_t* sp = d.sp;
-    const uint64_t T = (uint64_t)gridDim.x * kMcThreads;
-    const uint64_t me = (uint64_t)blockIdx.x * kMcThreads + threadIdx.x;
+    const uint32_t T = gridDim.x * kMcThreads, me = blockIdx.x * kMcThreads + threadIdx.x;
     const int colors = kParity ? 2 : a.classes[0] * a.classes[1] * a.classes[2];
-    unsigned long long my_att = 0, my_acc = 0, my_up = 0;
+    unsigned long long sum_att = 0, sum_acc = 0, sum_up = 0;
+    uint32_t my_att = 0, my_acc = 0, my_up = 0;  // of one sweep
+
+    struct Cells {              // the four cells of a thread in one pass
+        int cx, gi, y, z, par;
+        unsigned on;            // cells that attempt a change
+        uint32_t prop;          // proposals before the skip over the cell's own orientation
+        uint32_t nb[4];         // kNb == 2: byte j of nb[k]: bits 8 k .. 8 k + 7 of cell j's variant mask
+        uint64_t acc[4];        // acceptance numbers
+    };
+    struct Rows {               // what the trials read: the nine rows' eight bytes and the byte beside them
+        uint2 v[9];
+        uint8_t by[9];
+    };
+    // The cells of index i of colour c.
+    auto locate = [&](int c, uint64_t i, Cells& q) {
+        int cx = 0, cy = 0, cz = 0;
+        if (!kParity) {
+            cx = c % a.classes[0];
+            const int r = c / a.classes[0];
+            cy = r % a.classes[1];
+            cz = r / a.classes[1];
+        }
+        uint32_t ig, iy;
+        const uint32_t r = fast_divmod((uint32_t)i, d.div_gx[cx], ig);
+        const uint32_t iz = fast_divmod(r, d.div_cy[cy], iy);
+        q.cx = cx;
+        q.gi = (int)ig + d.g0[cx];
+        q.y = kParity ? (int)iy : class_coord((int)iy, cy, a.classes[1], a.ny);
+        q.z = kParity ? (int)iz : class_coord((int)iz, cz, a.classes[2], a.nz);
+        q.par = kParity ? (c + q.y + q.z + a.zoff) & 1 : cx & 1;
+    };
+    // Their draws (hashRand of the sweep and cell; they depend on no orientation).
+    auto draw = [&](uint64_t prefix, Cells& q) {
+        q.on = 0;
+        q.prop = 0;
+        uint32_t vm[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int x = 8 * q.gi + q.par + 2 * j;
+            const bool in = x >= d.xlo[q.cx] && x < d.xhi[q.cx];
+            const uint32_t g = (uint32_t)(in ? x : 0) + (uint32_t)a.nx * ((uint32_t)q.y + (uint32_t)a.ny * (uint32_t)q.z);
+            const uint64_t h = hash_index(prefix, g + a.gidx_base);
+            bool on = in;
+            if (kMobility) {
+                const uint64_t rr = hash_salt(h, kSaltMcMobility);
+                on = on && __dmul_rn((double)(rr >> 11), 1.0 / 9007199254740992.0) < (double)d.mob[g];
+            }
+            if (kNb == 2) vm[j] = d.mask[a.variants == 1 ? 0 : (int)fast_mod(hash_salt(h, kSaltNeighborhood), a.var_mod)];
+            q.on |= (unsigned)on << j;
+            q.prop |= mod_q(d, hash_salt(h, kSaltMcOrient)) << (8 * j);
+            q.acc[j] = d.uphill ? hash_salt(h, kSaltMcAccept) : 0;
+        }
+        if (kNb == 2) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                q.nb[k] = ((vm[0] >> 8 * k) & 0xFFu) | (((vm[1] >> 8 * k) & 0xFFu) << 8) | (((vm[2] >> 8 * k) & 0xFFu) << 16) |
+                          (((vm[3] >> 8 * k) & 0xFFu) << 24);
+        }
+    };
+    // All loads of the trials in one round, a missing row of the frame as the cells' own.
+    auto load = [&](const Cells& q, Rows& w) {
+        const uint8_t* row = d.sp + ((uint64_t)q.y + (uint64_t)a.ny * q.z) * (uint64_t)d.P8 + 8 + 8 * q.gi;
+        const int side = q.par ? 8 : -1;
+        int64_t oy[3], oz[3];
+        bool ky[3], kz[3];
+        mc_axis_nb(q.y, a.ny, a.per[1], d.P8, oy, ky);
+        mc_axis_nb(q.z, a.nz, a.per[2], (int64_t)d.P8 * a.ny, oz, kz);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            const int dy = i % 3, dz = i / 3;
+            if (kNb == 1 && dy != 1 && dz != 1) continue;
+            const uint8_t* p = row + (ky[dy] && kz[dz] ? oy[dy] + oz[dz] : 0);
+            w.v[i] = *reinterpret_cast<const uint2*>(p);
+            if (kNb != 1 || i == 4) w.by[i] = p[side];
+        }
+    };
+    // The trials (colorTrials, PottsMC.cpp:394-493).
+    auto trials_of = [&](const Cells& q, const Rows& rows, auto parity) {
+        const int par = decltype(parity)::value < 0 ? q.par : decltype(parity)::value;
+        if (!q.on) return;
+        my_att += __popc(q.on);
+        uint8_t* row = d.sp + ((uint64_t)q.y + (uint64_t)a.ny * q.z) * (uint64_t)d.P8 + 8 + 8 * q.gi;
+        // rows that exist: bytes of ones
+        const uint32_t wy[3] = {q.y > 0 || (a.per[1] && a.ny > 1) ? ~0u : 0u, ~0u, q.y < a.ny - 1 || (a.per[1] && a.ny > 1) ? ~0u : 0u};
+        const uint32_t wz[3] = {q.z > 0 || (a.per[2] && a.nz > 1) ? ~0u : 0u, ~0u, q.z < a.nz - 1 || (a.per[2] && a.nz > 1) ? ~0u : 0u};
+        // a frame that does not wrap: no left neighbour at x = 0, no right one at x = nx - 1
+        uint32_t ml = 0xFFFFFFFFu, mr = 0xFFFFFFFFu;
+        if (!a.per[0]) {
+            if (q.gi == 0 && par == 0) ml = 0xFFFFFF00u;
+            const int jr = a.nx - 1 - 8 * q.gi - par;
+            if ((jr & 1) == 0 && jr >= 0 && jr < 8) mr &= ~(0xFFu << (4 * jr));
+        }
+        // left, middle and right neighbours of the four cells in row i
+        auto words = [&](int i, uint32_t& left, uint32_t& mid, uint32_t& right) {
+            const uint32_t by = rows.by[i];
+            const uint32_t even = __byte_perm(rows.v[i].x, rows.v[i].y, 0x6420), odd = __byte_perm(rows.v[i].x, rows.v[i].y, 0x7531);
+            left = par ? even : __byte_perm(odd, by, 0x2104);   // bytes by, odd 0 .. 2
+            mid = par ? odd : even;
+            right = par ? __byte_perm(even, by, 0x4321) : odd;  // bytes even 1 .. 3, by
+        };
+        uint32_t lw, cur, rw;
+        words(4, lw, cur, rw);
+        // the proposals skip their cell's orientation: + 1 where proposal >= orientation, byte by byte
+        // (bit 7 of a - b with the borrow kept inside the byte, corrected where the top bits differ)
+        uint32_t prop;
+        {
+            const uint32_t pr = q.prop, dif = (pr | 0x80808080u) - (cur & 0x7F7F7F7Fu);
+            const uint32_t ge = (pr & ~cur) | (~(pr ^ cur) & dif);
+            prop = pr + ((ge >> 7) & 0x01010101u);
+        }
+        // bit 7 of each byte: the neighbour of that cell is unlike `v` (m: 0 bytes for missing neighbours)
+        auto unlike = [&](uint32_t w, uint32_t v, uint32_t m) -> uint32_t {
+            const uint32_t x = (w ^ v) & m;
+            return kWide ? ((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x : x + 0x7F7F7F7Fu;
+        };
+        Planes pa[3], pb[3];
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz) {
+            uint32_t sa[3], ca[3], sb[3], cb[3];
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy) {
+                sa[dy] = ca[dy] = sb[dy] = cb[dy] = 0;
+                if (kNb == 1 && dy != 1 && dz != 1) continue;
+                const int i = dy + 3 * dz;
+                const bool self = i == 4;
+                const uint32_t here = wy[dy] & wz[dz];
+                uint32_t w[3] = {lw, 0, rw}, ua[3] = {0, 0, 0}, ub[3] = {0, 0, 0};
+                if (!self && kNb == 1) w[1] = __byte_perm(rows.v[i].x, rows.v[i].y, par ? 0x7531 : 0x6420);
+                if (!self && kNb != 1) words(i, w[0], w[1], w[2]);
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) {
+                    if (self ? dx == 1 : kNb == 1 && dx != 1) continue;
+                    const uint32_t m = dx == 0 ? ml & here : dx == 2 ? mr & here : here;
+                    ua[dx] = unlike(w[dx], cur, m);
+                    ub[dx] = unlike(w[dx], prop, m);
+                    if (kNb == 2) {  // only the neighbours of the cell's variant
+                        const int bit = dx + 3 * dy + 9 * dz;
+                        const uint32_t of = q.nb[bit >> 3] << (7 - (bit & 7));
+                        ua[dx] &= of;
+                        ub[dx] &= of;
+                    }
+                }
+                add3(ua[0], ua[1], ua[2], sa[dy], ca[dy]);
+                add3(ub[0], ub[1], ub[2], sb[dy], cb[dy]);
+            }
+            pa[dz] = add_rows(sa, ca);
+            pb[dz] = add_rows(sb, cb);
+        }
+        // unlike neighbours of the orientations and of the proposals, a byte per cell
+        const uint32_t ua = add_planes(pa[0], pa[1], pa[2]), ub = add_planes(pb[0], pb[1], pb[2]);
+        unsigned took = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!((q.on >> j) & 1u)) continue;
+            // threshold << 11 (0: never), bit 0: not uphill, bit 1: uphill and always
+            const unsigned long long th = s_table[((ua >> (8 * j)) & 0xFFu) * kTableSide + ((ub >> (8 * j)) & 0xFFu)];
+            const bool free = ((uint32_t)th & 1u) != 0, accept = ((uint32_t)th & 3u) != 0 || q.acc[j] < th;
+            my_up += accept && !free ? 1u : 0u;
+            took |= (unsigned)accept << j;
+        }
+        if (!took) return;
+        my_acc += __popc(took);
+        if (8 * q.gi + 8 <= a.nx) {
+            // the eight bytes are this thread's alone in this pass: one store
+            const uint32_t m = ((took & 1u) | ((took & 2u) << 7) | ((took & 4u) << 14) | ((took & 8u) << 21)) * 0xFFu;
+            const uint32_t now = (prop & m) | (cur & ~m), even = par ? lw : now, odd = par ? now : rw;
+            *reinterpret_cast<uint2*>(row) = make_uint2(__byte_perm(even, odd, 0x5140), __byte_perm(even, odd, 0x7362));
+        } else {  // the last group of a row: the byte behind the cells is a frame column
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if ((took >> j) & 1u) row[par + 2 * j] = (uint8_t)(prop >> (8 * j));
+        }
+        if (a.per[0]) {  // the frame columns
+            if (q.gi == 0 && par == 0 && (took & 1u)) row[a.nx] = (uint8_t)prop;
+            const int jr = a.nx - 1 - 8 * q.gi - par;
+            if ((jr & 1) == 0 && jr >= 0 && jr < 8 && ((took >> (jr / 2)) & 1u)) row[-1 - 8 * q.gi] = (uint8_t)(prop >> (4 * jr));
+        }
+    };
+    // (the parity of x is the pass's own unless the colours are checkerboard parities)
+    auto trials = [&](const Cells& q, const Rows& rows) {
+        if constexpr (kParity) trials_of(q, rows, std::integral_constant<int, -1>{});
+        else if (q.par) trials_of(q, rows, std::integral_constant<int, 1>{});
+        else trials_of(q, rows, std::integral_constant<int, 0>{});
+    };
+    auto total_of = [&](int c) -> uint64_t {
+        int cx = 0, cy = 0, cz = 0;
+        if (!kParity) {
+            cx = c % a.classes[0];
+            const int r = c / a.classes[0];
+            cy = r % a.classes[1];
+            cz = r / a.classes[1];
+        }
+        return (uint64_t)d.gx[cx] * (uint32_t)d.cnt[1][cy] * (uint32_t)d.cnt[2][cz];
+    };
+
     bool ok = true;
     unsigned long long epoch = 0;
+    // the first cells of the next pass are drawn while the other blocks finish this one
+    Cells q;
+    if (sweeps > 0 && me < total_of(0)) {
+        locate(0, me, q);
+        draw(hash_prefix(a.seed, t0), q);
+    }
     for (int s = 0; s < sweeps && ok; ++s) {
         const uint64_t prefix = hash_prefix(a.seed, t0 + (uint32_t)s);
         for (int c = 0; c < colors && ok; ++c) {
-            int cx = 0, cy = 0, cz = 0;
-            if (!kParity) {
-                cx = c % a.classes[0];
-                const int r = c / a.classes[0];
-                cy = r % a.classes[1];
-                cz = r / a.classes[1];
+            const uint64_t total = total_of(c);
+            Rows rows;
+            if (me < total) {
+                load(q, rows);
+                trials(q, rows);
             }
-            const uint32_t nxc = (uint32_t)d.cnt[0][cx], nyc = (uint32_t)d.cnt[1][cy];
-            const uint64_t total = (uint64_t)nxc * nyc * (uint32_t)d.cnt[2][cz];
-            for (uint64_t i = me; i < total; i += T) {
-                uint32_t ix, iy;
-                const uint32_t r = fast_divmod((uint32_t)i, d.div[0][cx], ix);
-                const uint32_t iz = fast_divmod(r, d.div[1][cy], iy);
-                int x, y, z;
-                if (kParity) {
-                    y = (int)iy;
-                    z = (int)iz;
-                    x = 2 * (int)ix + ((c + y + z + a.zoff) & 1);
-                    if (x >= a.nx) continue;
-                } else {
-                    x = class_coord((int)ix, cx, a.classes[0], a.nx);
-                    y = class_coord((int)iy, cy, a.classes[1], a.ny);
-                    z = class_coord((int)iz, cz, a.classes[2], a.nz);
-                }
-                const uint32_t g = (uint32_t)x + (uint32_t)a.nx * ((uint32_t)y + (uint32_t)a.ny * (uint32_t)z);
-                const uint64_t h = hash_index(prefix, g + a.gidx_base);
-                if (kMobility) {
-                    const uint64_t rr = hash_salt(h, kSaltMcMobility);
-                    if (__dmul_rn((double)(rr >> 11), 1.0 / 9007199254740992.0) >= (double)d.mob[g]) continue;
-                }
-                ++my_att;
-                int var = 0;
-                if (kRandomNb) var = (int)fast_mod(hash_salt(h, kSaltNeighborhood), a.var_mod);
-                const int cur = (int)sp[g] + 1;
-                int prop = 1 + (int)fast_mod(hash_salt(h, kSaltMcOrient), a.qm1_mod);
-                if (prop >= cur) ++prop;
-                const uint32_t cb = (uint32_t)(cur - 1), pb = (uint32_t)(prop - 1);
-                int in_dom, same_a, same_b;
-                mc_count_block(a, sp, g, x, y, z, kMoore3 ? 0x7FFFFFFu & ~(1u << 13) : d.mask[var], 0x100u, cb, pb,
-                                      in_dom, same_a, same_b);
-                const unsigned long long th = s_table[(in_dom - same_a) * kTableSide + (in_dom - same_b)];
-                bool accept;
-                if (th >> 63) {
-                    accept = true;
-                } else {
-                    accept = th != 0 && (hash_salt(h, kSaltMcAccept) >> 11) < th;
-                    my_up += accept ? 1u : 0u;
-                }
-                if (accept) {
-                    d.sp[g] = (uint8_t)pb;
-                    ++my_acc;
-                }
+            for (uint64_t i = (uint64_t)me + T; i < total; i += T) {
+                locate(c, i, q);
+                load(q, rows);
+                draw(prefix, q);  // while the rows arrive
+                trials(q, rows);
             }
             mc_barrier_arrive(ctrl);
+            const bool last = c + 1 == colors;
+            const int nc = last ? 0 : c + 1;
+            if ((!last || s + 1 < sweeps) && me < total_of(nc)) {
+                locate(nc, me, q);
+                draw(last ? hash_prefix(a.seed, t0 + (uint32_t)s + 1u) : prefix, q);
+            }
             ok = mc_barrier_wait(ctrl, gridDim.x, ++epoch);
         }
+        sum_att += my_att, sum_acc += my_acc, sum_up += my_up;
+        my_att = my_acc = my_up = 0;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long ra = my_att, rc = my_acc, ru = my_up;
+    unsigned long long ra = sum_att, rc = sum_acc, ru = sum_up;
     for (int off = 16; off > 0; off >>= 1) {
         ra += __shfl_down_sync(0xFFFFFFFFu, ra, off);
         rc += __shfl_down_sync(0xFFFFFFFFu, rc, off);
@@ -952,7 +1223,8 @@ struct vca_mc {
     int profile_kernels = 0;
     std::vector<cudaEvent_t> prof_events;
     int slab_zoff = -1;                  // z slab of a taller grid (vca_mc_set_slab), -1: none
-    uint8_t* sp8 = nullptr;              // orientation - 1 per cell, for the whole-space sweeps (cap_n bytes)
+    uint8_t* sp8 = nullptr;              // orientation - 1 per cell, for the whole-space sweeps (grows only)
+    size_t sp8_cap = 0;
 };
 
 namespace {
@@ -1109,49 +1381,79 @@ vca_status sweeps_launch_shape(vca_mc* h, SweepsKernel kernel, McColors* col, in
     return VCA_OK;
 }
 
-using DenseKernel = void (*)(McArgs, McDense, int);
+using SpaceKernel = void (*)(McArgs, McSpace, int);
 
-template <bool kParity>
-DenseKernel dense_kernel_of(const vca_mc* h) {
-    const bool random_nb = h->nb_host.variants > 1;
-    const bool moore3 = !kParity && !random_nb && h->nb_host.count[0] == 26;
-    if (moore3) return h->mobility_on ? mc_dense_sweeps_kernel<true, false, false, true> : mc_dense_sweeps_kernel<false, false, false, true>;
-    if (h->mobility_on)
-        return random_nb ? mc_dense_sweeps_kernel<true, true, kParity, false> : mc_dense_sweeps_kernel<true, false, kParity, false>;
-    return random_nb ? mc_dense_sweeps_kernel<false, true, kParity, false> : mc_dense_sweeps_kernel<false, false, kParity, false>;
+template <bool kMobility, bool kWide>
+SpaceKernel space_kernel_of(const vca_mc* h) {
+    if (h->parity_colors) return mc_space_sweeps_kernel<kMobility, 1, true, kWide>;
+    switch (h->desc.neighborhood) {
+        case VCA_NB_MOORE: return mc_space_sweeps_kernel<kMobility, 0, false, kWide>;
+        case VCA_NB_VON_NEUMANN: return mc_space_sweeps_kernel<kMobility, 1, false, kWide>;
+        default: return mc_space_sweeps_kernel<kMobility, 2, false, kWide>;
+    }
+}
+SpaceKernel space_kernel_of(const vca_mc* h) {
+    if (h->desc.Q > 128) return h->mobility_on ? space_kernel_of<true, true>(h) : space_kernel_of<false, true>(h);
+    return h->mobility_on ? space_kernel_of<true, false>(h) : space_kernel_of<false, false>(h);
 }
 
-// The whole-space sweeps apply when every cell is in the domain and an orientation fits a byte.
-bool dense_applies(const vca_mc* h) {
+// Bytes of a row of the byte copy: 8 in front, the cells, 8 behind.
+int space_pitch(int nx) { return 8 + (nx + 7) / 8 * 8 + 8; }
+
+// A space that is one cell wide in x has the same order of cells as a plane of ny x nz: the sweeps see it
+// as that (the neighbourhood's offsets move down an axis).
+bool space_turned(const vca_mc* h) { return h->desc.nx == 1; }
+
+// The whole-space sweeps apply when every cell is in the domain, an orientation fits a byte, and the
+// rows are not so short that their frame columns outweigh them (below 6 cells).
+bool space_applies(const vca_mc* h) {
+    const int nx = space_turned(h) ? h->desc.ny : h->desc.nx;
     return !h->profile_kernels && h->slab_zoff < 0 && h->desc.Q <= 256 && !h->color_off.empty() &&
-           h->color_off.back() == h->n && h->n > 0;
+           h->color_off.back() == h->n && h->n > 0 && nx >= 6;
 }
 
-McDense dense_args(const vca_mc* h) {
-    McDense d;
+// The byte copy's shape and the colour classes; `a` becomes the sweep's view of a turned space.
+McSpace space_args(const vca_mc* h, McArgs& a) {
+    McSpace d;
     std::memset(&d, 0, sizeof(d));
-    d.sp = h->sp8;
-    d.mob = h->mobility_on ? h->mobility : nullptr;
-    const int dims[3] = {h->desc.nx, h->desc.ny, h->desc.nz};
-    for (int a = 0; a < 3; ++a) {
-        const int n = dims[a];
-        int* c = d.cnt[a];
-        c[0] = c[1] = c[2] = 1;
-        if (h->parity_colors) {
-            c[0] = a == 0 ? (n + 1) / 2 : n;
-        } else if (h->classes[a] == 1) {
-            c[0] = n;
-        } else if (h->classes[a] == 2) {
-            c[0] = (n + 1) / 2;
-            c[1] = n / 2;
-        } else {
-            c[0] = c[1] = (n - 1) / 2;
-            c[2] = 1;
+    for (int v = 0; v < 6; ++v) d.mask[v] = nb_mask(h->nb_host, v);
+    if (space_turned(h)) {
+        a.nx = h->desc.ny, a.ny = h->desc.nz, a.nz = 1;
+        for (int i = 0; i < 3; ++i) {
+            a.per[i] = i < 2 ? h->per[i + 1] : 0;
+            a.classes[i] = i < 2 ? h->classes[i + 1] : 1;
+        }
+        for (uint32_t& m : d.mask) {  // (0, dy, dz) -> (dy, dz, 0)
+            uint32_t to = 0;
+            for (int i = 0; i < 9; ++i)
+                if ((m >> (3 * i + 1)) & 1u) to |= 1u << (9 + i);
+            m = to;
         }
     }
-    for (int a = 0; a < 2; ++a)
-        for (int c = 0; c < 3; ++c) d.div[a][c] = make_fastdiv32((uint32_t)std::max(1, d.cnt[a][c]));
-    for (int v = 0; v < 6; ++v) d.mask[v] = nb_mask(h->nb_host, v);
+    d.sp = h->sp8;
+    d.mob = h->mobility_on ? h->mobility : nullptr;
+    d.P8 = space_pitch(a.nx);
+    const int dims[3] = {a.nx, a.ny, a.nz};
+    for (int ax = 0; ax < 3; ++ax) {
+        const int n = dims[ax], classes = h->parity_colors ? 1 : a.classes[ax];
+        int* c = d.cnt[ax];
+        c[0] = classes == 1 ? n : classes == 2 ? (n + 1) / 2 : (n - 1) / 2;
+        c[1] = classes == 1 ? 1 : n / 2;
+        c[2] = 1;
+    }
+    const int cx = h->parity_colors ? 1 : a.classes[0];
+    for (int c = 0; c < 3; ++c) {
+        d.xlo[c] = c == 2 ? a.nx - 1 : 0;
+        d.xhi[c] = cx == 3 && c < 2 ? a.nx - 1 : a.nx;
+        d.g0[c] = d.xlo[c] / 8;
+        d.gx[c] = (d.xhi[c] + 7) / 8 - d.g0[c];
+        d.div_gx[c] = make_fastdiv32((uint32_t)d.gx[c]);
+        d.div_cy[c] = make_fastdiv32((uint32_t)std::max(1, d.cnt[1][c]));
+    }
+    d.qm1 = (uint32_t)h->desc.Q - 1u;
+    d.qm1_inv = 0xFFFFFFFFu / d.qm1;
+    d.qm1_2p32 = (uint32_t)((1ULL << 32) % d.qm1);
+    d.uphill = h->desc.kT > 0.0;
     return d;
 }
 
@@ -1489,37 +1791,49 @@ vca_status vca_mc_sweep(vca_mc* h, int count, uint64_t* accepted) {
     };
     if (!h->profile_kernels) {
         // all sweeps in one cooperative launch (colour passes separated by grid barriers)
-        McColors col;
-        std::memset(&col, 0, sizeof(col));
-        col.colors = h->colors;
-        for (int c = 0; c <= h->colors; ++c) col.off[c] = h->color_off[c];
-        for (int v = 0; v < 6; ++v) col.mask[v] = nb_mask(h->nb_host, v);
-        int grid = 1;
-        size_t smem = 0;
-        SweepsKernel kernel = sweeps_kernel_of(h);
-        if (vca_status s = sweeps_launch_shape(h, kernel, &col, &grid, &smem)) return s;
-        const bool dense = dense_applies(h);
-        if (dense && !h->sp8) VCA_CUDA(cudaMalloc(&h->sp8, h->cap_n));
+        const bool space = space_applies(h);
         VCA_CUDA(cudaEventRecord(h->ev_a, h->stream));
-        if (count > 0 && dense) {
+        if (count > 0 && space) {
             // whole space: sweeps on the byte copy of the orientations, copied back after
-            const McDense d = dense_args(h);
-            DenseKernel dk = h->parity_colors ? dense_kernel_of<true>(h) : dense_kernel_of<false>(h);
+            McArgs va = a;
+            McSpace d = space_args(h, va);
+            const uint64_t rows = (uint64_t)va.ny * va.nz, bytes = (uint64_t)d.P8 * rows;
+            if (bytes > h->sp8_cap) {  // grows only
+                VCA_CUDA(cudaStreamSynchronize(h->stream));
+                cudaFree(h->sp8);
+                h->sp8 = nullptr;
+                h->sp8_cap = 0;
+                VCA_CUDA(cudaMalloc(&h->sp8, bytes));
+                h->sp8_cap = bytes;
+                d.sp = h->sp8;
+            }
+            SpaceKernel sk = space_kernel_of(h);
             int per_sm = 0;
-            VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dk, kMcThreads, 0));
-            const int dgrid = h->sms * std::max(1, per_sm);
-            const int blocks = grid_for(h->n, h->sms);
-            mc_pack8_kernel<<<blocks, 256, 0, h->stream>>>(h->spin, h->sp8, h->n);
+            VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sk, kMcThreads, 0));
+            // no more blocks than the largest colour has groups for
+            const uint64_t most = (uint64_t)d.gx[0] * (uint64_t)d.cnt[1][0] * (uint64_t)d.cnt[2][0];
+            const int sgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((most + kMcThreads - 1) / kMcThreads,
+                                                                           (uint64_t)h->sms * std::max(1, per_sm)));
+            const int blocks = grid_for(bytes / 8, h->sms);
+            mc_pack8_kernel<<<blocks, 256, 0, h->stream>>>(h->spin, h->sp8, va.nx, d.P8, rows);
             VCA_CUDA(cudaGetLastError());
             int n = count;
-            McDense dd = d;
-            void* args[] = {&a, &dd, &n};
-            if (vca_status s = barrier_reset(dgrid)) return s;
-            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)dk, dgrid, kMcThreads, args, 0, h->stream));
-            mc_unpack8_kernel<<<blocks, 256, 0, h->stream>>>(h->sp8, h->spin, h->n);
+            void* args[] = {&va, &d, &n};
+            if (vca_status s = barrier_reset(sgrid)) return s;
+            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)sk, sgrid, kMcThreads, args, 0, h->stream));
+            mc_unpack8_kernel<<<blocks, 256, 0, h->stream>>>(h->sp8, h->spin, va.nx, d.P8, rows);
             VCA_CUDA(cudaGetLastError());
             h->launches += 3;
         } else if (count > 0 && h->color_off.back() > 0) {
+            McColors col;
+            std::memset(&col, 0, sizeof(col));
+            col.colors = h->colors;
+            for (int c = 0; c <= h->colors; ++c) col.off[c] = h->color_off[c];
+            for (int v = 0; v < 6; ++v) col.mask[v] = nb_mask(h->nb_host, v);
+            int grid = 1;
+            size_t smem = 0;
+            SweepsKernel kernel = sweeps_kernel_of(h);
+            if (vca_status s = sweeps_launch_shape(h, kernel, &col, &grid, &smem)) return s;
             int n = count;
             void* args[] = {&a, &col, &n};
             if (vca_status s = barrier_reset(grid)) return s;
