@@ -178,7 +178,7 @@ __global__ __launch_bounds__(kFloodThreads, 1) void flood_kernel(const FloodArgs
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(&c->bar) : "memory");
                 if (v >= target) break;
-                if (spins > (1 << 26) || *(volatile unsigned*)&c->error) {
+                if (spins > (1 << 26) || ((spins & 1023) == 1023 && *(volatile unsigned*)&c->error)) {
                     ok = false;
                     break;
                 }
