@@ -1461,19 +1461,31 @@ __global__ void ca_seed_kernel(const __grid_constant__ CaKernelArgs k, const int
 using namespace vca;
 
 namespace vca {
+// The handle's step counter and stop state from the host mirror.
+static vca_status take_mirror(vca_ca* h) {
+    h->mirrored = true;
+    h->steps = (int)h->ctrl_host->steps;
+    h->stop = h->ctrl_host->stop;
+    if (h->ctrl_host->error) {
+        set_error("vca_ca: a bounded device wait (a tile copy or a grid barrier) ran out; the run was stopped");
+        return VCA_ERR_TIMEOUT;
+    }
+    return VCA_OK;
+}
 // Pull the control block to the host mirror.
 vca_status sync_ctrl(vca_ca* h) {
     ca_ctrl_snapshot_kernel<<<1, 32, 0, h->stream>>>(h->ctrl, h->ctrl_host_dev);
     VCA_CUDA(cudaGetLastError());
     VCA_CUDA(cudaStreamSynchronize(h->stream));
-    h->steps = (int)h->ctrl_host->steps;
-    h->stop = h->ctrl_host->stop;
-    if (h->ctrl_host->error) {
-        set_error("vca_ca: a bounded device wait (TMA tile copy) ran out; the run was stopped");
-        return VCA_ERR_TIMEOUT;
-    }
-    return VCA_OK;
+    return take_mirror(h);
 }
+// The same from a control block that a launch has already handed to the host.
+vca_status sync_ctrl(vca_ca* h, const CaCtrl& c) {
+    *h->ctrl_host = c;
+    return take_mirror(h);
+}
+// The mirror as it is when nothing has changed the control block since it was taken.
+vca_status know_ctrl(vca_ca* h) { return h->mirrored ? take_mirror(h) : sync_ctrl(h); }
 }  // namespace vca
 
 namespace {
@@ -1588,6 +1600,7 @@ vca_status tile_init(vca_ca* h, int steps_done) {
 
 // Totals and initial stop state of the current buffer, and what the handle's step kernels start from.
 vca_status init_state(vca_ca* h, int steps_done) {
+    h->mirrored = false;
     CaCtrl c;
     std::memset(&c, 0, sizeof(c));
     c.steps = (uint32_t)steps_done;
@@ -1729,6 +1742,7 @@ vca_status run_steps(vca_ca* h, int max_new_steps, bool until_stop) {
         return VCA_ERR_STATE;
     }
     if (h->stop != VCA_STOP_RUNNING) return VCA_OK;
+    h->mirrored = false;  // until the run has read its last control block
     if (h->front) return front_run(h, max_new_steps, until_stop);
     const CaKernelArgs k = make_args(h);
     if (until_stop && !h->profile_kernels) return run_graphs(h, k);
@@ -2380,7 +2394,7 @@ vca_status vca_ca_get_info(vca_ca* h, vca_ca_info* out) {
         return VCA_ERR_ARG;
     }
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     out->steps = h->steps;
     out->stop_reason = h->stop;
     out->lava_cells = h->ctrl_host->lava;
@@ -2397,7 +2411,7 @@ vca_status vca_ca_history(vca_ca* h, uint64_t* active, uint64_t* changed, int ca
     if (vca_status s = check(h)) return s;
     if (vca_status s = not_in_batch(h, "vca_ca_history")) return s;
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const int n = std::min(std::max(capacity, 0), h->steps);
     if (n > 0 && active) VCA_CUDA(cudaMemcpyAsync(active, h->hist_active, 8 * (size_t)n, cudaMemcpyDeviceToHost, h->stream));
     if (n > 0 && changed) VCA_CUDA(cudaMemcpyAsync(changed, h->hist_changed, 8 * (size_t)n, cudaMemcpyDeviceToHost, h->stream));
@@ -2411,7 +2425,7 @@ vca_status vca_ca_download(vca_ca* h, uint8_t* type, int32_t* flow_id, float* te
     if (vca_status s = check(h)) return s;
     if (vca_status s = not_in_batch(h, "vca_ca_download")) return s;
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const int cur = h->cur();
     if (type) if (vca_status s = get_plane(h, type, h->type[cur])) return s;
     if (flow_id) if (vca_status s = get_plane(h, flow_id, h->flow[cur])) return s;
@@ -2442,7 +2456,7 @@ vca_status vca_ca_flow_stats(vca_ca* h, int flows, uint64_t* lava, uint64_t* bas
         return VCA_ERR_ARG;
     }
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const size_t m = (size_t)flows + 1;
     if (3 * m > h->flow_sums_cap) {  // grows only
         VCA_CUDA(cudaStreamSynchronize(h->stream));
@@ -2524,6 +2538,7 @@ vca_status vca_ca_slab_stop(vca_ca* h, int stop_reason) {
     }
     VCA_CUDA(cudaSetDevice(h->device));
     const int32_t v = stop_reason;
+    h->mirrored = false;
     VCA_CUDA(cudaMemcpyAsync(&h->ctrl->stop, &v, sizeof(v), cudaMemcpyHostToDevice, h->stream));
     VCA_CUDA(cudaStreamSynchronize(h->stream));
     h->stop = stop_reason;
@@ -2535,7 +2550,7 @@ vca_status vca_ca_layers(vca_ca* h, void** type, void** flow_id, void** temp, vo
     if (vca_status s = check(h)) return s;
     if (vca_status s = not_in_batch(h, "vca_ca_layers")) return s;
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const int cur = h->cur();
     if (type) *type = h->type[cur];
     if (flow_id) *flow_id = h->flow[cur];
@@ -2561,7 +2576,7 @@ static vca_status layers_check(vca_ca* h, int z0, int types, int full, const voi
 
 static vca_status copy_layers(vca_ca* h, int z0, int types, int full, void* buf, bool to_buf) {
     VCA_CUDA(cudaSetDevice(h->device));
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const int cur = h->cur();
     if (!to_buf) h->front_listed = false;  // the copied layers may hold other LAVA cells
     const size_t L = (size_t)h->geom.P * h->geom.ny;
@@ -2626,7 +2641,7 @@ namespace vca {
 vca_status ca_view(vca_ca* h, CaView* v) {
     if (vca_status s = check(h)) return s;
     if (vca_status s = not_in_batch(h, "vca_mc_set_domain_from_ca / vca_mc_set_mobility_from_ca")) return s;
-    if (vca_status s = sync_ctrl(h)) return s;
+    if (vca_status s = know_ctrl(h)) return s;
     const int cur = h->cur();
     v->type = h->type[cur];
     v->solid = h->solid[cur];
@@ -2992,6 +3007,7 @@ vca_status vca_ca_batch_add(vca_ca_batch* b, vca_ca* h) {
     b->weight[(size_t)slot] = std::max<uint64_t>(1, h->front ? h->ctrl_host->front_n : h->ntiles);  // until its first status
     h->batch = b;
     h->batch_slot = slot;
+    h->mirrored = false;  // the batch steps it
     b->dirty = true;
     return VCA_OK;
 }

@@ -583,7 +583,10 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
             k.temp[pidx(k.g, x, y, z)] = te;
         }
     }
-    if (tid == 0) {
+    __syncthreads();
+    if (warp != 0) return;
+    bool last = false;
+    if (lane == 0) {
         if (bid == 0 && ok && t != t_first) {
             ctrl->steps = t;
             ctrl->stop = stop;
@@ -593,16 +596,17 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
         }
         unsigned left;
         asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(left) : "l"(&ctrl->front_exit) : "memory");
-        if (left == nblk - 1u) {  // the last block out: every block's totals are in
+        last = left == nblk - 1u;
+        if (last) {  // the last block out: every block's totals are in
             ctrl->front_exit = 0;
             if (ok && t != t_first) ctrl->lava = __ldcg(&k.hist_active[t - 1u]);
-            if (snap != nullptr) {
-                const uint32_t* from = reinterpret_cast<const uint32_t*>(ctrl);
-                volatile uint32_t* to = reinterpret_cast<volatile uint32_t*>(snap);
-                for (int i = 0; i < (int)(sizeof(CaCtrl) / sizeof(uint32_t)); ++i) to[i] = __ldcg(from + i);
-            }
         }
     }
+    if (!__shfl_sync(0xFFFFFFFFu, (int)last, 0) || snap == nullptr) return;
+    __syncwarp();
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(ctrl);
+    volatile uint32_t* to = reinterpret_cast<volatile uint32_t*>(snap);
+    for (int i = lane; i < (int)(sizeof(CaCtrl) / sizeof(uint32_t)); i += 32) to[i] = __ldcg(from + i);
 }
 
 __global__ __launch_bounds__(kFrontThreads, 1) void ca_front_kernel(const __grid_constant__ CaFrontArgs k, int steps,
@@ -778,9 +782,13 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
         const bool solo = n <= kFrontSolo;
         uint32_t most = solo && until_stop ? kFrontSolo : 0xFFFFFFFFu;
         CaCtrl* snap = h->ctrl_ring_dev + slot;
-        void* args[] = {&k, &steps, &most, &snap};
-        VCA_CUDA(cudaLaunchCooperativeKernel((const void*)ca_front_kernel, solo ? 1 : h->sms, kFrontThreads, args, 0, h->stream));
-        VCA_CUDA(cudaEventRecord(h->ring_ev[slot], h->stream));
+        if (solo) {
+            ca_front_kernel<<<1, kFrontThreads, 0, h->stream>>>(k, steps, most, snap);
+            VCA_CUDA(cudaGetLastError());
+        } else {
+            void* args[] = {&k, &steps, &most, &snap};
+            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)ca_front_kernel, h->sms, kFrontThreads, args, 0, h->stream));
+        }
         h->launches += 1;
         return VCA_OK;
     };
@@ -791,6 +799,7 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
         int pending = -1, slot = 0;
         for (;;) {
             if (vca_status s = launch(kFrontChunk, last.front_n, slot)) return s;
+            VCA_CUDA(cudaEventRecord(h->ring_ev[slot], h->stream));
             if (pending >= 0) {
                 VCA_CUDA(cudaEventSynchronize(h->ring_ev[pending]));
                 last = h->ctrl_ring[pending];
@@ -805,7 +814,8 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
     float ms = 0.f;
     VCA_CUDA(cudaEventElapsedTime(&ms, h->ev_a, h->ev_b));
     h->total_ms += ms;
-    return sync_ctrl(h);
+    if (!until_stop) last = h->ctrl_ring[0];
+    return sync_ctrl(h, last);
 }
 
 }  // namespace vca

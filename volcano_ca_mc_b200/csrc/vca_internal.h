@@ -230,6 +230,7 @@ struct vca_ca {
     vca::CaCtrl* ctrl = nullptr;
     vca::CaCtrl* ctrl_host = nullptr;   // pinned, host-mapped mirror
     vca::CaCtrl* ctrl_host_dev = nullptr;  // its device address
+    bool mirrored = false;              // the mirror is current and the stream idle
     uint32_t* tile_flags = nullptr;
     uint32_t* tile_mark[2] = {nullptr, nullptr};
     int8_t* desc_plane = nullptr;
@@ -281,6 +282,7 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop);
 int front_batch_grid(int sms);                                      // blocks of a batched launch, 0 on failure
 cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cudaStream_t stream);
 vca_status sync_ctrl(vca_ca* h);
+vca_status sync_ctrl(vca_ca* h, const CaCtrl& c);                   // from a block handed over by a launch
 // terrain.cu: heights and spill levels into their planes, ROCK columns
 vca_status terrain_apply(vca_ca* h, const int32_t* heights, int32_t lowest);
 }  // namespace vca
