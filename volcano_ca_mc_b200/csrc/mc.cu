@@ -14,11 +14,10 @@
 // (r >> 11) < ceil(p * 2^53); the thresholds are built on the host with the host's exp(), once
 // per (unlikeBefore, unlikeAfter) pair, and the device compares 64-bit integers.
 #include <cuda_runtime.h>
-#include <cub/device/device_select.cuh>
-#include <thrust/iterator/counting_iterator.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <type_traits>
@@ -49,8 +48,9 @@ struct McCtrl {
     unsigned long long uphill;
     unsigned long long energy_acc;
     unsigned long long sweep_accepted;  // accepted in the running sweep
-    unsigned long long bar_arrived;     // grid barrier of the fused sweep kernel: arrivals so far
+    unsigned long long bar_arrived;     // grid barrier of the cooperative launches: arrivals so far
                                         // (zeroed before each launch)
+    unsigned int cooling[4];            // mc_cooling_kernel: largest step, largest time, largest ~time
     int error;                          // bit 0: a bounded barrier wait ran out
     int pad;
 };
@@ -131,46 +131,135 @@ __device__ __forceinline__ void decode(const McArgs& a, uint32_t g, int& x, int&
 }
 
 // PottsMC::initialize (PottsMC.cpp:104-143): 1 + hashRand(seed, 0, g, McInit) % Q in the domain.
-__global__ void mc_init_kernel(McArgs a, const uint8_t* domain, uint64_t n) {
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        int32_t s = 0;
-        if (domain[g])
-            s = 1 + (int32_t)fast_mod(hash_salt(hash_index(hash_prefix(a.seed, 0), g + a.gidx_base), kSaltMcInit), a.q_mod);
-        a.spin[g] = s;
+__device__ __forceinline__ int32_t mc_first(const McArgs& a, uint64_t prefix, uint64_t g) {
+    return 1 + (int32_t)fast_mod(hash_salt(hash_index(prefix, g + a.gidx_base), kSaltMcInit), a.q_mod);
+}
+
+// A whole-space domain: every cell an orientation, four per thread.
+__global__ void mc_init_all_kernel(const __grid_constant__ McArgs a, uint64_t n) {
+    const uint64_t prefix = hash_prefix(a.seed, 0);
+    const uint64_t quads = (n + 3) / 4;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < quads; i += (uint64_t)gridDim.x * blockDim.x) {
+        int32_t s[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] = mc_first(a, prefix, 4 * i + j);
+        if (4 * i + 4 <= n) *reinterpret_cast<int4*>(a.spin + 4 * i) = make_int4(s[0], s[1], s[2], s[3]);
+        else
+            for (int j = 0; 4 * i + j < n; ++j) a.spin[4 * i + j] = s[j];
     }
 }
 
-// Cells of each colour in the domain (buildColors' class sizes, PottsMC.cpp:194-223).
-__global__ void mc_color_count_kernel(McArgs a, const uint8_t* domain, uint64_t n, int colors, unsigned long long* counts) {
-    __shared__ unsigned int s_cnt[28];
-    for (int c = threadIdx.x; c < 28; c += blockDim.x) s_cnt[c] = 0;
-    __syncthreads();
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        if (!domain[g]) continue;
-        int x, y, z;
-        decode(a, (uint32_t)g, x, y, z);
-        atomicAdd(&s_cnt[color_of(a, x, y, z)], 1u);
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < colors; c += blockDim.x)
-        if (s_cnt[c]) atomicAdd(&counts[c], (unsigned long long)s_cnt[c]);
-}
-
-struct ColorPred {
-    McArgs a;
+// The colour lists (buildColors, PottsMC.cpp:194-223) in three launches.  A block takes a contiguous run
+// of the space, 16 domain bytes per thread at a time: the first pass writes the orientations (0 outside
+// the domain) and counts the run's cells of each colour; the second, one block, turns the counts into
+// places (colour by colour, run by run); the third puts the cells there.  Within a run the order is the
+// atomics'; the trials of a colour do not depend on it.  Bounded by the bytes: 2 per cell read and 4
+// written.  vca_mc_initialize of 512 x 512 x 256 cells on one B200 against a count and a stream selection
+// per colour: 401 K in the domain 1.89 -> 0.24 ms, a whole space (now without lists) 2.7 -> 0.25 ms;
+// 256 x 256 x 128, 81 K 0.35 -> 0.07 ms.
+constexpr int kRunCells = 16 * kMcThreads;  // cells of one step of a block
+struct McRuns {
     const uint8_t* domain;
-    int color;
-    __device__ bool operator()(uint32_t g) const {
-        if (!domain[g]) return false;
-        int x, y, z;
-        decode(a, g, x, y, z);
-        return color_of(a, x, y, z) == color;
-    }
+    uint64_t n;
+    uint64_t per_block;      // cells of a block's run, a multiple of kRunCells
+    int colors;
+    uint32_t* counts;        // [color][block]: counts, then places
 };
-
-__global__ void mc_gather_mob_kernel(const uint32_t* list, const float* mob, float* out, uint64_t n) {
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
-        out[j] = mob[list[j]];
+template <class F>
+__device__ __forceinline__ void mc_each_domain_cell(const McRuns& r, F&& f) {
+    const uint64_t lo = blockIdx.x * r.per_block, hi = min(lo + r.per_block, r.n);
+    for (uint64_t base = lo + 16 * threadIdx.x; base < hi; base += kRunCells) {
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (base + 16 <= r.n) {
+            const uint4 v = *reinterpret_cast<const uint4*>(r.domain + base);
+            w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+        } else {
+            for (int j = 0; base + j < r.n; ++j) w[j >> 2] |= (uint32_t)r.domain[base + j] << (8 * (j & 3));
+        }
+        f(base, w);
+    }
+}
+__global__ __launch_bounds__(kMcThreads) void mc_runs_count_kernel(const __grid_constant__ McArgs a, const __grid_constant__ McRuns r,
+                                                                   int first) {
+    __shared__ uint32_t s_cnt[28];
+    if (threadIdx.x < 28) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t prefix = hash_prefix(a.seed, 0);
+    mc_each_domain_cell(r, [&](uint64_t base, const uint32_t w[4]) {
+        int32_t s[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            s[j] = 0;
+            if (((w[j >> 2] >> (8 * (j & 3))) & 0xFFu) == 0) continue;
+            if (first) s[j] = mc_first(a, prefix, base + j);
+            int x, y, z;
+            decode(a, (uint32_t)(base + j), x, y, z);
+            atomicAdd(&s_cnt[color_of(a, x, y, z)], 1u);
+        }
+        if (!first) return;
+        if (base + 16 <= r.n) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<int4*>(a.spin + base + 4 * q) = make_int4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (base + j < r.n) a.spin[base + j] = s[j];
+        }
+    });
+    __syncthreads();
+    if (threadIdx.x < r.colors) r.counts[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = s_cnt[threadIdx.x];
+}
+// Exclusive places of every (colour, block), and the colours' totals for the host (host-mapped).
+__global__ __launch_bounds__(1024) void mc_runs_place_kernel(uint32_t* counts, int colors, int blocks, volatile uint32_t* totals) {
+    __shared__ uint32_t s_warp[32];
+    __shared__ uint32_t s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_base = 0;
+    for (int c = 0; c < colors; ++c) {
+        __syncthreads();
+        const uint32_t first = s_base;
+        for (int b0 = 0; b0 < blocks; b0 += 1024) {
+            const int b = b0 + threadIdx.x;
+            uint32_t* at = counts + (uint64_t)c * blocks + b;
+            const uint32_t v = b < blocks ? *at : 0u;
+            uint32_t incl = v;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= off) incl += u;
+            }
+            __syncthreads();  // s_base and s_warp of the round before have been read
+            if (lane == 31) s_warp[warp] = incl;
+            __syncthreads();
+            uint32_t before = s_base;
+            for (int w = 0; w < warp; ++w) before += s_warp[w];
+            if (b < blocks) *at = before + incl - v;
+            __syncthreads();
+            if (threadIdx.x == 1023) s_base = before + incl;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) totals[c] = s_base - first;
+    }
+}
+__global__ __launch_bounds__(kMcThreads) void mc_runs_list_kernel(const __grid_constant__ McArgs a, const __grid_constant__ McRuns r,
+                                                                  const float* mob, uint32_t* list, float* list_mob) {
+    __shared__ uint32_t s_at[28];
+    if (threadIdx.x < r.colors) s_at[threadIdx.x] = r.counts[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x];
+    __syncthreads();
+    mc_each_domain_cell(r, [&](uint64_t base, const uint32_t w[4]) {
+        if (!(w[0] | w[1] | w[2] | w[3])) return;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (((w[j >> 2] >> (8 * (j & 3))) & 0xFFu) == 0) continue;
+            const uint32_t g = (uint32_t)(base + j);
+            int x, y, z;
+            decode(a, g, x, y, z);
+            const uint32_t at = atomicAdd(&s_at[color_of(a, x, y, z)], 1u);
+            list[at] = g;
+            if (mob != nullptr) list_mob[at] = mob[g];
+        }
+    });
 }
 
 // One colour of one MCS: colorTrials (PottsMC.cpp:394-448) for the list entries [0, count).
@@ -1187,7 +1276,7 @@ __global__ __launch_bounds__(kMcThreads) void mc_energy_kernel(McArgs a, const u
     const uint64_t prefix = hash_prefix(a.seed, a.ctrl->sweeps);
     unsigned long long mine = 0;
     for (uint64_t j = blockIdx.x * (uint64_t)kMcThreads + threadIdx.x; j < count; j += (uint64_t)gridDim.x * kMcThreads) {
-        const uint32_t g = list[j];
+        const uint32_t g = list ? list[j] : (uint32_t)j;  // no list: the whole space in order
         int x, y, z;
         decode(a, g, x, y, z);
         const int32_t s = a.spin[g];
@@ -1266,7 +1355,7 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
     const uint64_t i0 = blockIdx.x * (uint64_t)kMcThreads + threadIdx.x, T = (uint64_t)gridDim.x * kMcThreads;
     const int lane = threadIdx.x & 31;
     for (uint64_t j = i0; j < count; j += T) {
-        const uint32_t g = list[j];
+        const uint32_t g = list ? list[j] : (uint32_t)j;
         parent[g] = g;
         gsize[g] = 0;
         ghigh[g] = 0;
@@ -1274,7 +1363,7 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
     mc_barrier_arrive(a.ctrl);
     if (!mc_barrier_wait(a.ctrl, gridDim.x, 1)) return;
     for (uint64_t j = i0; j < count; j += T) {
-        const uint32_t g = list[j];
+        const uint32_t g = list ? list[j] : (uint32_t)j;
         const int32_t sg = a.spin[g];
         if (sg <= 0) continue;
         int x, y, z;
@@ -1305,7 +1394,7 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
     unsigned long long cells = 0, high = 0;
     for (uint64_t base = i0 - lane; base < count; base += T) {  // uniform over the warp
         const uint64_t j = base + lane;
-        const uint32_t g = j < count ? list[j] : 0u;
+        const uint32_t g = j < count ? (list ? list[j] : (uint32_t)j) : 0u;
         const bool on = j < count && a.spin[g] > 0;
         uint32_t r = 0xFFFFFFFFu;
         bool up = false;
@@ -1328,7 +1417,7 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
     unsigned long long v[5] = {0, 0, 0, 0, 0};  // grains; high ones, their cells; low ones, their cells
     unsigned long long largest = 0, hl = 0, ll = 0;
     for (uint64_t j = i0; j < count; j += T) {
-        const uint32_t g = list[j];
+        const uint32_t g = list ? list[j] : (uint32_t)j;
         if (a.spin[g] <= 0 || parent[g] != g) continue;
         const unsigned long long sz = __ldcg(&gsize[g]);
         ++v[0];
@@ -1373,76 +1462,130 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
     }
 }
 
-// CoolingMobility (engine/src/mc/CoolingMobility.cpp) on the device.
+// CoolingMobility (engine/src/mc/CoolingMobility.cpp) on the device.  W cells of a row per thread (W
+// divides nx, so that a group is aligned in the pitched planes and in the unpitched domain).
+template <int W>
+struct Cells8 {  // W bytes
+    uint8_t v[W];
+};
+template <int W>
+__device__ __forceinline__ Cells8<W> load_bytes(const uint8_t* p) {
+    Cells8<W> c;
+    if constexpr (W == 16) *reinterpret_cast<uint4*>(c.v) = *reinterpret_cast<const uint4*>(p);
+    else if constexpr (W == 4) *reinterpret_cast<uint32_t*>(c.v) = *reinterpret_cast<const uint32_t*>(p);
+    else c.v[0] = *p;
+    return c;
+}
+template <int W>
 __global__ void mc_domain_from_ca_kernel(const uint8_t* type, int nx, int P, uint64_t rows, uint8_t* domain) {
-    const uint64_t n = (uint64_t)nx * rows;
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = g / nx;
-        const int x = (int)(g - r * nx);
-        const uint8_t t = type[r * P + x];
-        domain[g] = (t == kBasalt || t == kLava) ? 1 : 0;  // basaltDomain (CoolingMobility.cpp:8-14)
+    const uint32_t per_row = (uint32_t)nx / W;
+    const uint64_t n = per_row * rows;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t r = i / per_row;
+        const uint32_t x = W * (uint32_t)(i - r * per_row);
+        __align__(16) Cells8<W> c = load_bytes<W>(type + r * (uint64_t)P + x);
+#pragma unroll
+        for (int j = 0; j < W; ++j) c.v[j] = (c.v[j] == kBasalt || c.v[j] == kLava) ? 1 : 0;  // basaltDomain (CoolingMobility.cpp:8-14)
+        uint8_t* to = domain + r * (uint64_t)nx + x;
+        if constexpr (W == 16) *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(c.v);
+        else if constexpr (W == 4) *reinterpret_cast<uint32_t*>(to) = *reinterpret_cast<const uint32_t*>(c.v);
+        else *to = c.v[0];
     }
 }
 
-// endStep: largest solidStep / arrivalStep in the domain (CoolingMobility.cpp:16-25).
-__global__ void mc_end_step_kernel(const uint16_t* solid, const uint16_t* arrival, const uint8_t* domain, int nx, int P,
-                                   uint64_t rows, unsigned int* end_step) {
-    unsigned m = 0;
-    const uint64_t n = (uint64_t)nx * rows;
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        if (!domain[g]) continue;
-        const uint64_t r = g / nx;
-        const uint64_t p = r * P + (g - r * nx);
-        m = max(m, (unsigned)max(solid[p], arrival[p]));
+struct McCooling {
+    const uint8_t* type;
+    const uint16_t* solid;
+    const uint16_t* arrival;
+    const uint8_t* domain;
+    int nx, P;
+    uint64_t rows;
+    double mobility_min;
+    unsigned int* sums;      // largest step, largest time, largest ~time (all zero before the launch)
+    float* mobility;
+    McCtrl* ctrl;
+};
+// fromCooling in one cooperative launch: endStep, the largest solidStep / arrivalStep in the domain
+// (CoolingMobility.cpp:16-25); liquidTime (32-45) and its range (timeRange, 47-56); normalize (58-74):
+// mobilityMin + (1 - mobilityMin) * (t - tMin) / (tMax - tMin) in double, each operation rounded once (no
+// contraction), then to float.  Bounded by the 4 bytes per cell it writes; a call for 512 x 512 x 256
+// cells took 0.52 ms with three launches over a plane of times, 0.20 ms with this one.
+template <int W>
+__global__ __launch_bounds__(kMcThreads) void mc_cooling_kernel(const __grid_constant__ McCooling m) {
+    const uint32_t per_row = (uint32_t)m.nx / W;
+    const uint64_t n = per_row * m.rows, T = (uint64_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    auto any = [](const Cells8<W>& d) {
+        unsigned v = 0;
+#pragma unroll
+        for (int j = 0; j < W; ++j) v |= d.v[j];
+        return v != 0;
+    };
+    unsigned last = 0;
+    for (uint64_t i = i0; i < n; i += T) {
+        __align__(16) const Cells8<W> d = load_bytes<W>(m.domain + i * W);
+        if (!any(d)) continue;
+        const uint64_t r = i / per_row, p = r * (uint64_t)m.P + W * (i - r * per_row);
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (d.v[j]) last = max(last, (unsigned)max(m.solid[p + j], m.arrival[p + j]));
     }
-    m = __reduce_max_sync(0xFFFFFFFFu, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(end_step, m);
-}
-
-// liquidTime (CoolingMobility.cpp:32-45) and its range (timeRange, 47-56): mm[0] = min, mm[1] = max.
-__global__ void mc_time_range_kernel(const uint8_t* type, const uint16_t* solid, const uint16_t* arrival,
-                                     const uint8_t* domain, int nx, int P, uint64_t rows, const unsigned int* end_step,
-                                     unsigned int* time, unsigned int* mm) {
-    unsigned lo = 0xFFFFFFFFu, hi = 0;
-    const unsigned end = *end_step;
-    const uint64_t n = (uint64_t)nx * rows;
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        unsigned tm = 0;
-        if (domain[g]) {
-            const uint64_t r = g / nx;
-            const uint64_t p = r * P + (g - r * nx);
-            const unsigned s = type[p] == kBasalt ? solid[p] : end;
-            const unsigned ar = arrival[p];
-            tm = s > ar ? s - ar : 0;
-            lo = min(lo, tm);
-            hi = max(hi, tm);
-        }
-        time[g] = tm;
+    last = __reduce_max_sync(0xFFFFFFFFu, last);
+    if ((threadIdx.x & 31) == 0 && last) atomicMax(&m.sums[0], last);
+    mc_barrier_arrive(m.ctrl);
+    if (!mc_barrier_wait(m.ctrl, gridDim.x, 1)) return;
+    const unsigned end = __ldcg(&m.sums[0]);
+    auto time_of = [&](uint64_t p) -> unsigned {
+        const unsigned s = m.type[p] == kBasalt ? m.solid[p] : end, ar = m.arrival[p];
+        return s > ar ? s - ar : 0;
+    };
+    unsigned hi = 0, nlo = 0;
+    for (uint64_t i = i0; i < n; i += T) {
+        __align__(16) const Cells8<W> d = load_bytes<W>(m.domain + i * W);
+        if (!any(d)) continue;
+        const uint64_t r = i / per_row, p = r * (uint64_t)m.P + W * (i - r * per_row);
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (d.v[j]) {
+                const unsigned t = time_of(p + j);
+                hi = max(hi, t);
+                nlo = max(nlo, ~t);
+            }
     }
-    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
     hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    nlo = __reduce_max_sync(0xFFFFFFFFu, nlo);
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&mm[0], lo);
-        atomicMax(&mm[1], hi);
+        if (hi) atomicMax(&m.sums[1], hi);
+        if (nlo) atomicMax(&m.sums[2], nlo);
     }
-}
-
-// normalize (CoolingMobility.cpp:58-74): mobilityMin + (1 - mobilityMin) * (t - tMin) / (tMax - tMin)
-// in double, each operation rounded once (no contraction), then to float.
-__global__ void mc_normalize_kernel(const unsigned int* time, const uint8_t* domain, const unsigned int* mm,
-                                    double mobility_min, uint64_t n, float* mobility) {
-    const unsigned lo = mm[0], hi = mm[1];
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
-        float m = 0.0f;
-        if (domain[g]) {
-            if (hi == lo) {
-                m = 1.0f;
-            } else {
-                const double norm = __ddiv_rn((double)(time[g] - lo), (double)(hi - lo));
-                m = __double2float_rn(__dadd_rn(mobility_min, __dmul_rn(__dsub_rn(1.0, mobility_min), norm)));
+    mc_barrier_arrive(m.ctrl);
+    if (!mc_barrier_wait(m.ctrl, gridDim.x, 2)) return;
+    hi = __ldcg(&m.sums[1]);
+    const unsigned lo = ~__ldcg(&m.sums[2]);
+    for (uint64_t i = i0; i < n; i += T) {
+        __align__(16) const Cells8<W> d = load_bytes<W>(m.domain + i * W);
+        __align__(16) float v[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) v[j] = 0.0f;
+        if (any(d)) {
+            const uint64_t r = i / per_row, p = r * (uint64_t)m.P + W * (i - r * per_row);
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                if (!d.v[j]) continue;
+                if (hi == lo) {
+                    v[j] = 1.0f;
+                } else {
+                    const double norm = __ddiv_rn((double)(time_of(p + j) - lo), (double)(hi - lo));
+                    v[j] = __double2float_rn(__dadd_rn(m.mobility_min, __dmul_rn(__dsub_rn(1.0, m.mobility_min), norm)));
+                }
             }
         }
-        mobility[g] = m;
+        float* to = m.mobility + i * W;
+        if constexpr (W >= 4) {
+#pragma unroll
+            for (int q = 0; q < W / 4; ++q) reinterpret_cast<float4*>(to)[q] = reinterpret_cast<const float4*>(v)[q];
+        } else {
+            *to = v[0];
+        }
     }
 }
 
@@ -1478,11 +1621,11 @@ struct vca_mc {
     bool initialized = false;
     int sms = 148;
     // set-up buffers, allocated on first use and kept (no cudaMalloc / cudaFree per call)
-    size_t list_cap = 0;                 // cells that list / list_mob can hold
-    unsigned int* scratch = nullptr;     // mobility: [end, min, max] + time[n]
-    void* cub_temp = nullptr;
-    size_t cub_temp_bytes = 0;
-    unsigned long long* d_count = nullptr;  // 28 colour counts
+    uint32_t* run_counts = nullptr;      // [color][block] of the list build
+    uint32_t* totals_host = nullptr;     // pinned, host-mapped: cells per colour (behind gacc_host)
+    uint32_t* totals_host_dev = nullptr; // its device address
+    bool domain_all = false;             // every cell is in the domain
+    bool listed = false;                 // the colour lists are built (a whole space needs them rarely)
     uint32_t* gparent = nullptr;         // grain statistics: parent, size, high count per cell (n each)
     uint32_t* gsize = nullptr;
     uint32_t* ghigh = nullptr;
@@ -1573,9 +1716,7 @@ void mc_free(vca_mc* h) {
     cudaFree(h->list_mob);
     cudaFree(h->table);
     cudaFree(h->ctrl);
-    cudaFree(h->scratch);
-    cudaFree(h->cub_temp);
-    cudaFree(h->d_count);
+    cudaFree(h->run_counts);
     cudaFree(h->gparent);
     cudaFree(h->gsize);
     cudaFree(h->ghigh);
@@ -1679,6 +1820,55 @@ int space_pitch(int nx) { return 8 + (nx + 7) / 8 * 8 + 8; }
 // A space that is one cell wide in x has the same order of cells as a plane of ny x nz: the sweeps see it
 // as that (the neighbourhood's offsets move down an axis).
 bool space_turned(const vca_mc* h) { return h->desc.nx == 1; }
+
+// Cells of colour c when every cell is in the domain.
+uint64_t whole_color_size(const vca_mc* h, int c) {
+    if (h->parity_colors) return c == 0 ? (h->n + 1) / 2 : h->n / 2;  // (x + y + z) & 1
+    const int dims[3] = {h->desc.nx, h->desc.ny, h->desc.nz};
+    uint64_t size = 1;
+    for (int a = 0; a < 3; ++a) {
+        const int k = c % h->classes[a], n = dims[a];
+        c /= h->classes[a];
+        size *= (uint64_t)(h->classes[a] == 1 ? n : h->classes[a] == 2 ? (n + 1 - k) / 2 : k == 2 ? 1 : (n - 1) / 2);
+    }
+    return size;
+}
+
+// The colour lists of the domain; with `first` also the first orientations (vca_mc_initialize), else the
+// orientations stay (a whole space whose lists are wanted after all).
+vca_status build_lists(vca_mc* h, bool first) {
+    const uint64_t steps = (h->n + kRunCells - 1) / kRunCells;
+    const uint64_t cap_steps = (h->cap_n + kRunCells - 1) / kRunCells, most = (uint64_t)h->sms * 16;
+    // sized for the capacity, so that later, larger spaces on a resident handle allocate nothing
+    if (!h->run_counts) VCA_CUDA(cudaMalloc(&h->run_counts, sizeof(uint32_t) * 28 * std::max<uint64_t>(1, std::min(cap_steps, most))));
+    if (!h->list || (h->mobility_on && !h->list_mob)) {
+        cudaFree(h->list);
+        cudaFree(h->list_mob);
+        h->list = nullptr;
+        h->list_mob = nullptr;
+        VCA_CUDA(cudaMalloc(&h->list, 4 * std::max<uint64_t>(h->cap_n, 1)));
+        VCA_CUDA(cudaMalloc(&h->list_mob, 4 * std::max<uint64_t>(h->cap_n, 1)));
+    }
+    const McArgs a = mc_args(h);
+    McRuns r;
+    std::memset(&r, 0, sizeof(r));
+    r.domain = h->domain;
+    r.n = h->n;
+    r.per_block = (steps + most - 1) / most * kRunCells;
+    r.colors = h->colors;
+    r.counts = h->run_counts;
+    const int blocks = (int)((h->n + r.per_block - 1) / r.per_block);
+    mc_runs_count_kernel<<<blocks, kMcThreads, 0, h->stream>>>(a, r, first ? 1 : 0);
+    mc_runs_place_kernel<<<1, 1024, 0, h->stream>>>(h->run_counts, h->colors, blocks, h->totals_host_dev);
+    mc_runs_list_kernel<<<blocks, kMcThreads, 0, h->stream>>>(a, r, h->mobility_on ? h->mobility : nullptr, h->list, h->list_mob);
+    VCA_CUDA(cudaGetLastError());
+    VCA_CUDA(cudaStreamSynchronize(h->stream));
+    h->color_off.assign((size_t)h->colors + 1, 0);
+    for (int c = 0; c < h->colors; ++c) h->color_off[(size_t)c + 1] = h->color_off[(size_t)c] + h->totals_host[c];
+    h->listed = true;
+    return VCA_OK;
+}
+vca_status want_lists(vca_mc* h) { return h->listed ? VCA_OK : build_lists(h, false); }
 
 // The whole-space sweeps apply when every cell is in the domain, an orientation fits a byte, and the
 // rows are not so short that their frame columns outweigh them (below 6 cells).
@@ -1890,13 +2080,16 @@ vca_status vca_mc_create(const vca_mc_desc* d, vca_mc** out) {
         (e = cudaMalloc(&h->table, 8 * kTableSide * kTableSide)) != cudaSuccess ||
         (e = cudaMalloc(&h->ctrl, sizeof(McCtrl))) != cudaSuccess)
         return fail(cuda_fail(e, "cudaMalloc"));
-    // one pinned block: the mirror of the control block, then that of the grain statistics
+    // one pinned block: the mirror of the control block, that of the grain statistics, colour totals
     static_assert(sizeof(McCtrl) % alignof(GrainAcc) == 0, "GrainAcc follows McCtrl");
-    if ((e = cudaHostAlloc(&h->ctrl_host, sizeof(McCtrl) + sizeof(GrainAcc), cudaHostAllocMapped)) != cudaSuccess ||
+    if ((e = cudaHostAlloc(&h->ctrl_host, sizeof(McCtrl) + sizeof(GrainAcc) + 28 * sizeof(uint32_t), cudaHostAllocMapped)) !=
+            cudaSuccess ||
         (e = cudaHostGetDevicePointer(&h->ctrl_host_dev, h->ctrl_host, 0)) != cudaSuccess)
         return fail(cuda_fail(e, "cudaHostAlloc (mapped)"));
     h->gacc_host = reinterpret_cast<GrainAcc*>(h->ctrl_host + 1);
     h->gacc_host_dev = reinterpret_cast<GrainAcc*>(h->ctrl_host_dev + 1);
+    h->totals_host = reinterpret_cast<uint32_t*>(h->gacc_host + 1);
+    h->totals_host_dev = reinterpret_cast<uint32_t*>(h->gacc_host_dev + 1);
     if ((e = cudaEventCreate(&h->ev_a)) != cudaSuccess || (e = cudaEventCreate(&h->ev_b)) != cudaSuccess)
         return fail(cuda_fail(e, "cudaEventCreate"));
     const char* prof = std::getenv("VCA_PROFILE_KERNELS");
@@ -1928,8 +2121,8 @@ vca_status vca_mc_footprint(const vca_mc_desc* d, uint64_t* bytes) {
     }
     if (vca_status s = mc_validate(d, "vca_mc_footprint")) return s;
     const uint64_t n = (uint64_t)d->nx * d->ny * d->nz;
-    // spin 4 + domain 1 + mobility 4 + mobility scratch 4 + colour lists 8 + grain labels 12 bytes per cell,
-    // the list-selection scratch (bounded by 4 bytes per cell), tables and counters
+    // spin 4 + domain 1 + mobility 4 + colour lists 8 + grain labels 12 bytes per cell, the byte copy of the
+    // orientations (at most 4 bytes per cell), the list build's counts, tables and counters
     *bytes = 37 * n + 8 * kTableSide * kTableSide + sizeof(McCtrl) + 8 * 28 + sizeof(NbTable) + 4096;
     return VCA_OK;
 }
@@ -1945,6 +2138,7 @@ vca_status vca_mc_set_domain(vca_mc* h, const uint8_t* in_domain) {
     } else {
         VCA_CUDA(cudaMemsetAsync(h->domain, 1, h->n, h->stream));
     }
+    h->domain_all = in_domain == nullptr;
     h->domain_set = true;
     h->initialized = false;
     return VCA_OK;
@@ -1980,9 +2174,13 @@ vca_status vca_mc_set_domain_from_ca(vca_mc* h, vca_ca* ca) {
     }
     VCA_CUDA(cudaSetDevice(h->device));
     VCA_CUDA(cudaStreamSynchronize(v.stream));
-    mc_domain_from_ca_kernel<<<h->sms * 8, 256, 0, h->stream>>>(v.type, v.nx, v.P, (uint64_t)v.ny * v.nz, h->domain);
+    const uint64_t rows = (uint64_t)v.ny * v.nz;
+    if (v.nx % 16 == 0) mc_domain_from_ca_kernel<16><<<h->sms * 8, 256, 0, h->stream>>>(v.type, v.nx, v.P, rows, h->domain);
+    else if (v.nx % 4 == 0) mc_domain_from_ca_kernel<4><<<h->sms * 8, 256, 0, h->stream>>>(v.type, v.nx, v.P, rows, h->domain);
+    else mc_domain_from_ca_kernel<1><<<h->sms * 8, 256, 0, h->stream>>>(v.type, v.nx, v.P, rows, h->domain);
     VCA_CUDA(cudaGetLastError());
     VCA_CUDA(cudaStreamSynchronize(h->stream));
+    h->domain_all = false;
     h->domain_set = true;
     h->initialized = false;
     return VCA_OK;
@@ -2003,20 +2201,30 @@ vca_status vca_mc_set_mobility_from_ca(vca_mc* h, vca_ca* ca, double mobility_mi
     VCA_CUDA(cudaSetDevice(h->device));
     VCA_CUDA(cudaStreamSynchronize(v.stream));
     if (!h->mobility) VCA_CUDA(cudaMalloc(&h->mobility, 4 * h->cap_n));
-    if (!h->scratch) VCA_CUDA(cudaMalloc(&h->scratch, 4 * (3 + h->cap_n)));
-    unsigned int* scratch = h->scratch;  // [end, min, max] + time[n]
-    const unsigned int init[3] = {0u, 0xFFFFFFFFu, 0u};
-    VCA_CUDA(cudaMemcpyAsync(scratch, init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
-    const uint64_t rows = (uint64_t)v.ny * v.nz;
-    const int blocks = h->sms * 8;
-    mc_end_step_kernel<<<blocks, 256, 0, h->stream>>>(v.solid, v.arrival, h->domain, v.nx, v.P, rows, scratch);
-    mc_time_range_kernel<<<blocks, 256, 0, h->stream>>>(v.type, v.solid, v.arrival, h->domain, v.nx, v.P, rows, scratch,
-                                                        scratch + 3, scratch + 1);
-    mc_normalize_kernel<<<blocks, 256, 0, h->stream>>>(scratch + 3, h->domain, scratch + 1, mobility_min, h->n, h->mobility);
-    cudaError_t e = cudaGetLastError();
-    cudaError_t e2 = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "mobility kernels");
-    if (e2 != cudaSuccess) return cuda_fail(e2, "mobility kernels");
+    McCooling m;
+    std::memset(&m, 0, sizeof(m));
+    m.type = v.type;
+    m.solid = v.solid;
+    m.arrival = v.arrival;
+    m.domain = h->domain;
+    m.nx = v.nx;
+    m.P = v.P;
+    m.rows = (uint64_t)v.ny * v.nz;
+    m.mobility_min = mobility_min;
+    m.sums = h->ctrl->cooling;
+    m.mobility = h->mobility;
+    m.ctrl = h->ctrl;
+    const int w = v.nx % 16 == 0 ? 16 : v.nx % 4 == 0 ? 4 : 1;
+    const void* kernel = w == 16 ? (const void*)mc_cooling_kernel<16> : w == 4 ? (const void*)mc_cooling_kernel<4>
+                                                                              : (const void*)mc_cooling_kernel<1>;
+    int per_sm = 0;
+    VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMcThreads, 0));
+    const int grid = (int)std::min<uint64_t>((h->n / w + kMcThreads - 1) / kMcThreads, (uint64_t)h->sms * std::max(1, std::min(per_sm, 4)));
+    static_assert(offsetof(McCtrl, cooling) == offsetof(McCtrl, bar_arrived) + 8, "one memset clears both");
+    VCA_CUDA(cudaMemsetAsync(&h->ctrl->bar_arrived, 0, 8 + sizeof(h->ctrl->cooling), h->stream));
+    void* args[] = {&m};
+    VCA_CUDA(cudaLaunchCooperativeKernel(kernel, grid, kMcThreads, args, 0, h->stream));
+    VCA_CUDA(cudaStreamSynchronize(h->stream));
     h->mobility_set = true;
     h->mobility_on = use_in_dynamics != 0;
     h->initialized = false;
@@ -2042,54 +2250,15 @@ vca_status vca_mc_initialize(vca_mc* h) {
         return VCA_ERR_STATE;
     }
     VCA_CUDA(cudaSetDevice(h->device));
-    McArgs a = mc_args(h);
-    mc_init_kernel<<<h->sms * 8, 256, 0, h->stream>>>(a, h->domain, h->n);
-    VCA_CUDA(cudaGetLastError());
-    // Colour lists, colour by colour, globalIndex ascending inside a colour (PottsMC.cpp:194-223):
-    // count the cells of each colour, then select each colour into its place of one list.
-    if (!h->d_count) VCA_CUDA(cudaMalloc(&h->d_count, 8 * 28));
-    VCA_CUDA(cudaMemsetAsync(h->d_count, 0, 8 * 28, h->stream));
-    mc_color_count_kernel<<<h->sms * 8, 256, 0, h->stream>>>(a, h->domain, h->n, h->colors, h->d_count);
-    VCA_CUDA(cudaGetLastError());
-    std::vector<unsigned long long> counts((size_t)h->colors, 0);
-    VCA_CUDA(cudaMemcpyAsync(counts.data(), h->d_count, 8 * (size_t)h->colors, cudaMemcpyDeviceToHost, h->stream));
-    VCA_CUDA(cudaStreamSynchronize(h->stream));
-    h->color_off.assign((size_t)h->colors + 1, 0);
-    uint64_t total = 0;
-    for (int c = 0; c < h->colors; ++c) {
-        h->color_off[c] = total;
-        total += counts[c];
-    }
-    h->color_off[h->colors] = total;
-    if (total > h->list_cap || (h->mobility_on && !h->list_mob)) {
-        cudaFree(h->list);
-        cudaFree(h->list_mob);
-        h->list = nullptr;
-        h->list_mob = nullptr;
-        h->list_cap = std::max<uint64_t>(std::max<uint64_t>(total, h->cap_n), 1);  // once per handle
-        VCA_CUDA(cudaMalloc(&h->list, 4 * h->list_cap));
-        VCA_CUDA(cudaMalloc(&h->list_mob, 4 * h->list_cap));
-    }
-    ColorPred pred{a, h->domain, 0};
-    thrust::counting_iterator<uint32_t> it(0);
-    size_t temp_bytes = 0;
-    // sized for the capacity, so that later, larger spaces on a resident handle allocate nothing
-    VCA_CUDA(cub::DeviceSelect::If(nullptr, temp_bytes, it, h->list, h->d_count, (int64_t)h->cap_n, pred, h->stream));
-    if (temp_bytes > h->cub_temp_bytes) {
-        cudaFree(h->cub_temp);
-        h->cub_temp = nullptr;
-        VCA_CUDA(cudaMalloc(&h->cub_temp, temp_bytes));
-        h->cub_temp_bytes = temp_bytes;
-    }
-    for (int c = 0; c < h->colors; ++c) {
-        if (counts[c] == 0) continue;
-        pred.color = c;
-        VCA_CUDA(cub::DeviceSelect::If(h->cub_temp, temp_bytes, it, h->list + h->color_off[c], h->d_count + c, (int64_t)h->n, pred,
-                                       h->stream));
-    }
-    if (h->mobility_on && total) {
-        mc_gather_mob_kernel<<<grid_for(total, h->sms), 256, 0, h->stream>>>(h->list, h->mobility, h->list_mob, total);
+    h->listed = false;
+    if (h->domain_all && h->slab_zoff < 0) {
+        // a whole space: the colours' sizes are known, and its sweeps, energy and grains need no lists
+        mc_init_all_kernel<<<h->sms * 8, 256, 0, h->stream>>>(mc_args(h), h->n);
         VCA_CUDA(cudaGetLastError());
+        h->color_off.assign((size_t)h->colors + 1, 0);
+        for (int c = 0; c < h->colors; ++c) h->color_off[(size_t)c + 1] = h->color_off[(size_t)c] + whole_color_size(h, c);
+    } else if (vca_status s = build_lists(h, true)) {
+        return s;
     }
     VCA_CUDA(cudaMemsetAsync(h->ctrl, 0, sizeof(McCtrl), h->stream));
     VCA_CUDA(cudaStreamSynchronize(h->stream));
@@ -2145,6 +2314,8 @@ vca_status vca_mc_sweep(vca_mc* h, int count, uint64_t* accepted) {
             VCA_CUDA(cudaGetLastError());
             h->launches += 3;
         } else if (count > 0 && h->color_off.back() > 0) {
+            if (vca_status s = want_lists(h)) return s;
+            a = mc_args(h);
             McColors col;
             std::memset(&col, 0, sizeof(col));
             col.colors = h->colors;
@@ -2201,6 +2372,8 @@ vca_status vca_mc_sweep(vca_mc* h, int count, uint64_t* accepted) {
         if (accepted) *accepted = h->ctrl_host->sweep_accepted;
         return VCA_OK;
     }
+    if (vca_status s = want_lists(h)) return s;
+    a = mc_args(h);
     VCA_CUDA(cudaEventRecord(h->ev_a, h->stream));
     const bool random_nb = h->nb_host.variants > 1;
     size_t ev_used = 0;
@@ -2299,7 +2472,7 @@ vca_status vca_mc_grains(vca_mc* h, int moore, double mobility_threshold, vca_mc
         VCA_CUDA(cudaMemsetAsync(acc, 0, sizeof(GrainAcc), h->stream));
         VCA_CUDA(cudaMemsetAsync(&h->ctrl->bar_arrived, 0, sizeof(unsigned long long), h->stream));
         const int grid = (int)std::min<uint64_t>((total + kMcThreads - 1) / kMcThreads, (uint64_t)h->sms * h->grain_per_sm);
-        const uint32_t* list = h->list;
+        const uint32_t* list = h->listed ? h->list : nullptr;  // none: every cell in order
         volatile GrainAcc* out = h->gacc_host_dev;
         void* args[] = {&a, &list, &total, &moore, &mob, &mobility_threshold, &h->gparent, &h->gsize, &h->ghigh, &acc, &out};
         VCA_CUDA(cudaLaunchCooperativeKernel((const void*)mc_grains_kernel, grid, kMcThreads, args, 0, h->stream));
@@ -2344,7 +2517,7 @@ vca_status vca_mc_energy(vca_mc* h, double* energy) {
     VCA_CUDA(cudaMemsetAsync(&h->ctrl->energy_acc, 0, 8, h->stream));
     const uint64_t total = h->color_off.back();
     const bool forward = h->nb_host.variants == 1;
-    if (total) mc_energy_kernel<<<grid_for(total, h->sms), kMcThreads, 0, h->stream>>>(mc_args(h), h->list, total, forward);
+    if (total) mc_energy_kernel<<<grid_for(total, h->sms), kMcThreads, 0, h->stream>>>(mc_args(h), h->listed ? h->list : nullptr, total, forward);
     h->launches += total ? 1 : 0;
     VCA_CUDA(cudaGetLastError());
     if (vca_status s_ = mc_sync(h)) return s_;
@@ -2399,6 +2572,7 @@ vca_status vca_mc_color_pass(vca_mc* h, int color) {
         return VCA_ERR_ARG;
     }
     VCA_CUDA(cudaSetDevice(h->device));
+    if (vca_status s = want_lists(h)) return s;
     const McArgs a = mc_args(h);
     const uint64_t b = h->color_off[color], cnt = h->color_off[color + 1] - b;
     const int grid = grid_for(cnt, h->sms);
