@@ -117,6 +117,38 @@ def test_scattered_states_match_oracle(case):
     ca.close()
 
 
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 512, 513, 37888, 37889, 40000, 40001, 148 * 1024 + 1])
+@pytest.mark.parametrize("mode", ["lava", "classic"])
+def test_list_lengths_at_the_edges_of_the_launch_shapes(n, mode):
+    """Runs from n LAVA cells of a dozen flows, packed so that most votes count many flows: one block, blocks
+    with a slot per thread, blocks that stream, and lists that outgrow the launch they started in."""
+    nx, ny, nz = (40, 24, 12) if n < 1000 else (80, 64, 48)
+    p = _params(nx, ny, nz, "moore", "periodic", 12, 6 + n, eruption_steps=4, mode=mode)
+    rng = np.random.default_rng(n)
+    cells = 2 * n if mode == "lava" else min(2 * n + 8, nx * ny * nz)
+    at = rng.choice(min(cells, nx * ny * nz), size=n, replace=False)
+    kind = np.zeros(nx * ny * nz, np.uint8)
+    kind[at] = 2
+    flow, temp = np.zeros(kind.size, np.int32), np.zeros(kind.size, np.float32)
+    flow[at] = rng.integers(1, 13, size=n)
+    temp[at] = rng.uniform(805, 840, size=n)
+    zero = np.zeros(kind.size, np.uint16)
+    s = O.CaState(nx, ny, nz, kind, flow, temp, zero, zero)
+    spill = np.zeros(nx * ny, np.int32) if mode == "lava" else None
+    ca = capi.LavaCA(p)
+    ca.set_state(s.type, s.flow, s.temp, s.solid, s.arrival, spill, [], steps_done=0)
+    op, vt = C.oracle_params(p), O.vent_table([])
+    for t in range(12):
+        s, counts = O.ca_step(op, t, s, spill, vt)
+        stop = O.ca_stop_after(op, t + 1, counts)
+        if stop:
+            break
+    ca.run()
+    assert (ca.info().steps, ca.info().stop_reason) == (t + 1, stop)
+    assert C.state_diff(s, ca.download()) == ""
+    ca.close()
+
+
 def test_more_solidifying_cells_than_a_block_gathers():
     """Most of a 786 000-cell block of LAVA solidifies in one step."""
     nx, ny, nz = 128, 128, 48

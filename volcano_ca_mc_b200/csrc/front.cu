@@ -26,15 +26,20 @@
 //
 // What bounds a step: with few cells (up to some 10^5) the latency of its chains -- list entry, types,
 // the barrier's release and poll, mark, source temperatures, slot of the new cell, the second barrier --
-// some 7 us with all SMs and 6 us in one block, whose barriers are __syncthreads; above that the list
+// some 7 us with all SMs and 5 us in one block, whose barriers are __syncthreads; above that the list
 // stream (9 bytes per LAVA cell from L2).  Against the tile schedule on one B200: 1024 x 1024 x 256,
-// 800 steps, up to 1.0 M LAVA cells 208 -> 15.3 ms; 256 x 256 x 128, 400 steps 14.9 -> 3.4 ms;
-// 512 x 1 x 256, 300 steps 8.1 -> 2.1 ms; classic 100^3, 70 steps 2.4 -> 1.4 ms; ten mixed jobs in a
-// batch 19.8 -> 6.2 ms.
+// 800 steps, up to 1.0 M LAVA cells 208 -> 13.8 ms; 256 x 256 x 128, 400 steps 14.9 -> 2.8 ms;
+// 512 x 1 x 256, 300 steps 8.1 -> 1.54 ms; classic 100^3, 70 steps 2.4 -> 1.2 ms; ten mixed jobs in a
+// batch 19.8 -> 6.1 ms.  Three forms brought the last part of it (mid: 256 x 256 x 128, 3.3 -> 2.8 ms):
+// slots held in registers while each thread has at most one; a block's births counted in shared memory, so
+// that each block takes its slots of the list with one atomic; and votes among five and more sources of
+// several flows by a warp, one lane per source (one thread counting them in local arrays held up the second
+// barrier of every step with such a cell).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <string>
 
@@ -53,18 +58,22 @@ constexpr int kWordBits = 10;         // barrier words count blocks in 10-bit fi
 constexpr unsigned kWordMask = (1u << kWordBits) - 1u;
 
 // Shared lists of a block of kThreads threads.  The queue is emptied when it is full; candidates and
-// solidifying slots that do not fit are listed in global memory.
+// solidifying slots that do not fit are listed in global memory, births that do not fit one by one.
 template <int kThreads>
 struct FrontShared {
     static constexpr int kQueue = 2 * kThreads, kCand = 4 * kThreads, kSolid = kThreads;
-    unsigned nqueue, ncand, nsolid, active, changed, born;
+    unsigned nqueue, ncand, nsolid, active, changed, born, base;
     unsigned long long word;    // the barrier word all blocks have arrived at, 0: gave up
-    uint32_t q_slot[kQueue];    // phase A: slots that look around (bit 31: vent)
-    uint32_t q_cell[kQueue];    // their cells; phase B: cells whose type changed
+    // phase A: the slots that look around (bit 31: vent), or with resident slots their threads; their cells
+    // and temperatures.  Phase B: the cells born in this step
+    uint32_t q_slot[kQueue];
+    uint32_t q_cell[kQueue];
     float q_temp[kQueue];
     uint32_t cand[kCand], solid[kSolid];
+    uint8_t flags[kThreads];    // resident slots: the flags of each thread's slot
 };
 constexpr uint32_t kVentBit = 1u << 31;
+constexpr uint32_t kRun = 8;          // consecutive slots of a block
 
 __device__ __forceinline__ void front_decode(const CaFrontArgs& k, uint32_t c, int& x, int& y, int& z) {
     uint32_t ux, uy;
@@ -132,7 +141,7 @@ __device__ __forceinline__ void front_emit(const CaFrontArgs& k, S& s, uint32_t*
 // (l % 3 - 1, l / 3 - 1) of it; lane 4 is the cell's own column.  Everything a lane needs short of a
 // fall of more than two cells comes in one round of loads.
 template <int kThreads>
-__device__ __forceinline__ void front_look_lava(const CaFrontArgs& k, FrontShared<kThreads>& s, uint32_t* over, unsigned nq) {
+__device__ __forceinline__ void front_look_lava(const CaFrontArgs& k, FrontShared<kThreads>& s, uint32_t* over, unsigned nq, bool resident) {
     const CaGeom& g = k.g;
     const int lane = threadIdx.x & 31, l = lane & 15, sh = lane & 16;
     const int i = l < 9 ? l : 4;
@@ -193,8 +202,9 @@ __device__ __forceinline__ void front_look_lava(const CaFrontArgs& k, FrontShare
         if (on && own) {
             const uint32_t qs = s.q_slot[j];
             if (any) k.temp[q] = s.q_temp[j];  // what the votes read
-            k.flags[qs & ~kVentBit] = (qs & kVentBit ? kFrontVent : 0) | (any ? 0 : kFrontIdle) |
-                                      (!below_air && airs == 0 && !can_pond ? kFrontQuiet : 0);
+            const uint8_t fl = (qs & kVentBit ? kFrontVent : 0) | (any ? 0 : kFrontIdle) |
+                               (!below_air && airs == 0 && !can_pond ? kFrontQuiet : 0);
+            *(resident ? s.flags + (qs & ~kVentBit) : k.flags + (qs & ~kVentBit)) = fl;
         }
     }
 }
@@ -202,7 +212,7 @@ __device__ __forceinline__ void front_look_lava(const CaFrontArgs& k, FrontShare
 // Phase A for the queued grain cells of a classic grid: every AIR cell of the neighbourhood, lane l at
 // the offsets l and l + 16.
 template <int kThreads>
-__device__ __forceinline__ void front_look_classic(const CaFrontArgs& k, FrontShared<kThreads>& s, uint32_t* over, unsigned nq) {
+__device__ __forceinline__ void front_look_classic(const CaFrontArgs& k, FrontShared<kThreads>& s, uint32_t* over, unsigned nq, bool resident) {
     const CaGeom& g = k.g;
     const int lane = threadIdx.x & 31, l = lane & 15, sh = lane & 16;
     for (unsigned base = 2 * (threadIdx.x >> 5); base < nq; base += 2 * (kThreads / 32)) {
@@ -224,78 +234,139 @@ __device__ __forceinline__ void front_look_classic(const CaFrontArgs& k, FrontSh
         const bool any = ((__ballot_sync(0xFFFFFFFFu, emit[0] || emit[1]) >> sh) & 0xFFFFu) != 0;
 #pragma unroll
         for (int r = 0; r < 2; ++r) front_emit(k, s, over, emit[r], lane, cx[r], cy[r], cz[r], 26 - (l + 16 * r));
-        if (on && l == 0) k.flags[s.q_slot[j]] = any ? 0 : kFrontQuiet;  // no AIR around: for good
+        if (on && l == 0) *(resident ? s.flags + s.q_slot[j] : k.flags + s.q_slot[j]) = any ? 0 : kFrontQuiet;  // no AIR around: for good
     }
 }
 
-// The vote among the sources `m` of a candidate in full (CandidateVote, CaRules.hpp:127-183).
-template <class V>
-__device__ __forceinline__ void front_tally(const CaFrontArgs& k, int x, int y, int z, uint32_t m, V& v) {
+// r % n for 1 <= n <= 26, r = hashRand(seed, t, idx, TieBreak), by the halves of r: 2^32 is (2^32 - 1) % n + 1
+// modulo n.
+__device__ __forceinline__ unsigned front_tie(uint64_t prefix, uint64_t cell, unsigned n) {
+    const uint64_t h = hash_salt(hash_index(prefix, cell), kSaltTieBreak);
+    return (((uint32_t)(h >> 32) % n) * (0xFFFFFFFFu % n + 1u) + (uint32_t)h % n) % n;
+}
+
+// One source of a candidate at (x, y, z): bit i of its mark.
+template <bool kClassic>
+__device__ __forceinline__ void front_source(const CaFrontArgs& k, int x, int y, int z, int i, int32_t& flow, float& temp) {
     const CaGeom& g = k.g;
-    v.n = 0;
-    for (; m; m &= m - 1) {
-        const int i = __ffs(m) - 1;
-        const int64_t q = pidx(g, axis_at(x, i % 3 - 1, g.nx), axis_at(y, i / 3 % 3 - 1, g.ny), axis_at(z, i / 9 - 1, g.nz));
-        v.add(k.flow[q], k.classic ? 0.0f : __fsub_rn(k.temp[q], i >= 18 ? k.cool_fall : k.cool_lateral));
-    }
-}
-__device__ __noinline__ void front_vote(const CaFrontArgs& k, int x, int y, int z, uint32_t m, uint64_t prefix, uint64_t cell,
-                                        int32_t* flow, float* temp) {
-    SmallVote v;
-    v.over = false;
-    front_tally(k, x, y, z, m, v);
-    if (!v.over) {
-        v.pick(prefix, cell, flow, temp);
-        return;
-    }
-    Vote w;  // five or more distinct flowIds
-    front_tally(k, x, y, z, m, w);
-    w.pick(prefix, cell, flow, temp);
+    const int64_t q = pidx(g, axis_at(x, i % 3 - 1, g.nx), axis_at(y, i / 3 % 3 - 1, g.ny), axis_at(z, i / 9 - 1, g.nz));
+    flow = k.flow[q];
+    // the source wrote its temperature of this step there; one above falls, the others spread
+    temp = kClassic ? 0.0f : __fsub_rn(k.temp[q], i >= 18 ? k.cool_fall : k.cool_lateral);
 }
 
-// Phase B for one candidate: returns true when it becomes LAVA with (nf, nt).
+// The vote among five and more sources `m` of several flows (CandidateVote, CaRules.hpp:127-183), a warp
+// for the candidate, lane i for source i; the winner in every lane.
+template <bool kClassic>
+__device__ __forceinline__ void front_vote(const CaFrontArgs& k, uint32_t c, uint32_t m, uint32_t t, int lane, int32_t& flow,
+                                           float& temp) {
+    int x, y, z;
+    front_decode(k, c, x, y, z);
+    const bool have = (m >> lane) & 1u;
+    int32_t fl = 0;
+    float te = 0.0f;
+    if (have) front_source<kClassic>(k, x, y, z, lane, fl, te);
+    const unsigned alike = __match_any_sync(0xFFFFFFFFu, fl) & m;
+    const bool lead = have && lane == __ffs(alike) - 1;
+    const int votes = lead ? __popc(alike) : 0, best = __reduce_max_sync(0xFFFFFFFFu, votes);
+    const unsigned tied = __ballot_sync(0xFFFFFFFFu, lead && votes == best), ties = __popc(tied);
+    // ties: the (r % ties)-th smallest tied id
+    const unsigned want = ties > 1 ? front_tie(hash_prefix(k.seed, t), c, ties) : 0u;
+    unsigned rank = 0;
+    for (unsigned r = tied; r; r &= r - 1) rank += __shfl_sync(0xFFFFFFFFu, fl, __ffs(r) - 1) < fl;
+    const unsigned won = __ballot_sync(0xFFFFFFFFu, lead && votes == best && rank == want);
+    const int src = __ffs(won) - 1;
+    flow = __shfl_sync(0xFFFFFFFFu, fl, src);
+    const unsigned of = __shfl_sync(0xFFFFFFFFu, alike, src);
+    temp = __shfl_sync(0xFFFFFFFFu, te, src);
+    for (unsigned r = of; r; r &= r - 1) temp = fmaxf(temp, __shfl_sync(0xFFFFFFFFu, te, __ffs(r) - 1));
+}
+
+// Phase B for one candidate: returns true when it becomes LAVA with (nf, nt); `hard` gets its sources when
+// five or more of several flows have to be counted (front_vote; the result is then false).
+template <bool kClassic>
 __device__ __forceinline__ bool front_decide(const CaFrontArgs& k, uint32_t c, int x, int y, int z, int64_t p, uint32_t t,
-                                             int32_t& nf, float& nt) {
-    const CaGeom& g = k.g;
+                                             int32_t& nf, float& nt, uint32_t& hard) {
     const uint32_t m = atomicExch(k.mark + p, 0u);
     const int var =
         k.variants == 1 ? 0 : (int)fast_mod(hash_salt(hash_index(hash_prefix(k.seed, t), c), kSaltNeighborhood), k.var_mod);
     const uint32_t use = m & k.vmask[var];
     if (!use) return false;
-    // sources of one flow need no vote: its highest temperature decides
-    bool same = true, first = true;
-    for (uint32_t r = use; r;) {
-        int32_t fl[4];
-        float te[4];
-        unsigned got = 0;
+    // four sources a round; the slots past the last one hold the first again
+    const int n = __popc(use);
+    int32_t fl[4];
+    float te[4];
+    uint32_t r = use;
+    bool same = true;
+    auto fetch = [&]() {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            fl[q] = 0;
-            te[q] = 0.0f;
-            if (r) {
-                const int i = __ffs(r) - 1;
-                r &= r - 1;
-                got |= 1u << q;
-                const int64_t sp = pidx(g, axis_at(x, i % 3 - 1, g.nx), axis_at(y, i / 3 % 3 - 1, g.ny), axis_at(z, i / 9 - 1, g.nz));
-                fl[q] = k.flow[sp];
-                // the source wrote its temperature of this step there; one above falls, the others spread
-                if (!k.classic) te[q] = __fsub_rn(k.temp[sp], i >= 18 ? k.cool_fall : k.cool_lateral);
-            }
+            fl[q] = q ? fl[0] : nf;
+            te[q] = q ? te[0] : nt;
+            if (!r) continue;
+            front_source<kClassic>(k, x, y, z, __ffs(r) - 1, fl[q], te[q]);
+            r &= r - 1;
         }
-        if (first) {
-            nf = fl[0];
-            nt = te[0];
-            first = false;
-        }
+    };
+    auto fold = [&]() {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if ((got >> q) & 1u) {
-                same = same && fl[q] == nf;
-                nt = fmaxf(nt, te[q]);
+        for (int q = 0; q < 4; ++q) {
+            same = same && fl[q] == nf;
+            nt = fmaxf(nt, te[q]);
+        }
+    };
+    fetch();
+    nf = fl[0];
+    nt = te[0];
+    fold();
+    // sources of one flow need no vote: its highest temperature decides
+    if (n > 4) {
+        while (r) {
+            fetch();
+            fold();
+        }
+        if (!same) {
+            hard = use;
+            return false;
+        }
+    } else if (!same) {
+        // the vote among two to four: most votes; ties: the (r % ties)-th smallest tied id
+        int votes[4], best = 0;
+        float most[4];
+        bool lead[4];  // the first source of its flow
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            votes[i] = 0;
+            most[i] = te[i];
+            lead[i] = i < n;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool alike = j < n && fl[j] == fl[i];
+                votes[i] += alike;
+                if (alike) most[i] = fmaxf(most[i], te[j]);
+                if (alike && j < i) lead[i] = false;
             }
+            if (lead[i]) best = max(best, votes[i]);
+        }
+        unsigned ties = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lead[i] = lead[i] && votes[i] == best;
+            ties += lead[i];
+        }
+        const unsigned want = ties > 1 ? front_tie(hash_prefix(k.seed, t), c, ties) : 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            unsigned rank = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) rank += lead[j] && fl[j] < fl[i];
+            if (lead[i] && rank == want) {
+                nf = fl[i];
+                nt = most[i];
+            }
+        }
     }
-    if (!same) front_vote(k, x, y, z, use, hash_prefix(k.seed, t), c, &nf, &nt);
-    return k.classic || nt >= k.solidus;
+    return kClassic || nt >= k.solidus;
 }
 
 // Thread 0's half of the barrier of a grid's `nblk` blocks: adds `add` (one arrival in the low field) to
@@ -329,7 +400,12 @@ __device__ __forceinline__ void front_stamp(const CaFrontArgs& k, uint32_t c, in
 
 // Up to `steps` steps of one grid by its `nblk` blocks (block `bid`), until its stop rule holds or its
 // list has grown beyond `most` slots.
-template <int kThreads>
+//
+// The list goes round the blocks in runs of 8 slots, a sector of each array: the cells that look around
+// lie together (the last ones born first of all) and are shared out.  While the list is no longer than the
+// launch has threads, a slot is resident in its thread: its cell and temperature stay in registers, its flags in shared memory, so that a step starts with one load (an idle cell's stamp)
+// instead of three dependent ones.  A longer list is streamed, four slots per thread.
+template <int kThreads, bool kClassic>
 __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kThreads>& s, uint32_t bid, uint32_t nblk, int steps,
                                            uint32_t most, CaCtrl* snap) {
     using S = FrontShared<kThreads>;
@@ -342,96 +418,149 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
     uint64_t air = ctrl->air, visited = 0;
     int stop = VCA_STOP_RUNNING;
     bool ok = true;
+    // the resident slot of this thread, once the list reaches it
+    bool resident = n <= T, have = false, dying = false;
+    const uint32_t my_slot = ((uint32_t)(tid / kRun) * nblk + bid) * kRun + tid % kRun;
+    uint32_t my_cell = 0, my_col = 0;
+    float my_temp = 0.0f;
     if (tid == 0) s.nqueue = s.ncand = s.nsolid = s.active = s.changed = s.born = 0;
     __syncthreads();
+    auto column = [&](uint32_t cell) -> uint32_t {
+        uint32_t x, y;
+        const uint32_t r = fast_divmod(cell, k.div_nx, x);
+        fast_divmod(r, k.div_ny, y);
+        return x + (uint32_t)k.g.nx * y;
+    };
+    auto stamp_type = [&](uint32_t c) {
+        for (int i = 0; i < 9; ++i) front_stamp(k, c, i, t);
+    };
+    // the resident slots back into the list
+    auto write_back = [&]() {
+        if (!have) return;
+        k.flags[my_slot] = s.flags[tid];
+        if (!kClassic) k.ltemp[my_slot] = my_temp;
+    };
     while (t - t_first < (uint32_t)steps && stop == VCA_STOP_RUNNING && n <= most) {
         uint32_t* over = ctrl->front_over[t % 3u];
         unsigned my_active = 0, my_changed = 0;
-        // ---- phase A.  One LAVA cell of the list: its temperature; returns whether it may look around.
-        auto cool = [&](uint32_t slot, unsigned fl, float& te) -> bool {
-            if (fl & kFrontDead) return false;
-            if (k.classic) {
-                ++my_active;
-            } else {
-                const bool vent = (fl & kFrontVent) != 0;
-                if (slot < prev) te = front_cool(k, te, vent, (int64_t)t - 1);  // the update of the last step
-                const float next = front_cool(k, te, vent, t);
-                if (next < k.solidus) {
-                    ++my_changed;
-                    const unsigned at = atomicAdd(&s.nsolid, 1u);
-                    if (at < (unsigned)S::kSolid) s.solid[at] = slot;
-                    else k.work[k.work_cap - 1u - atomicAdd(&over[1], 1u)] = slot;
-                } else {
-                    ++my_active;
-                    my_changed += next != te;
-                }
-            }
-            return !(fl & kFrontQuiet);
-        };
-        // An idle cell looks only if the last step changed a type around its column.
-        auto stale = [&](uint32_t cell) -> bool {
-            uint32_t x, y;
-            const uint32_t r = fast_divmod(cell, k.div_nx, x);
-            fast_divmod(r, k.div_ny, y);
-            return k.stamp[x + (uint32_t)k.g.nx * y] == t - 1u;
-        };
-        auto push = [&](uint32_t slot, unsigned fl, uint32_t cell, float te) -> bool {
-            const unsigned at = atomicAdd(&s.nqueue, 1u);
-            if (at >= (unsigned)S::kQueue) return false;
-            s.q_slot[at] = slot | (fl & kFrontVent ? kVentBit : 0u);
-            s.q_cell[at] = cell;
-            s.q_temp[at] = te;
-            return true;
-        };
+        if (resident && n > T) {  // outgrown: the same blocks go on with the same runs from memory
+            write_back();
+            resident = have = false;
+            __syncthreads();
+        }
         auto look = [&]() {
             __syncthreads();
             const unsigned nq = min(s.nqueue, (unsigned)S::kQueue);
-            if (k.classic) front_look_classic(k, s, over, nq);
-            else front_look_lava(k, s, over, nq);
+            if (kClassic) front_look_classic(k, s, over, nq, resident);
+            else front_look_lava(k, s, over, nq, resident);
         };
-        // The list goes round the blocks in runs of 32 slots: the cells that look around lie together
-        // (the last ones born first of all) and are shared out.
-        if (n <= T) {
-            const uint32_t slot = ((uint32_t)warp * nblk + bid) * 32u + lane;
-            if (slot < n) {
-                const unsigned fl = k.flags[slot];
-                const uint32_t cell = k.idx[slot];
-                float te = k.classic ? 0.0f : k.ltemp[slot];
-                const bool may = cool(slot, fl, te);
-                if (!k.classic) k.ltemp[slot] = te;
-                if (may && (!(fl & kFrontIdle) || stale(cell))) push(slot, fl, cell, te);  // kQueue >= kThreads
+        // ---- phase A
+        if (resident) {
+            unsigned fl = 0;
+            uint32_t seen = t - 1u;
+            if (have) {
+                fl = s.flags[tid];
+                if ((fl & (kFrontIdle | kFrontQuiet | kFrontDead)) == kFrontIdle) seen = k.stamp[my_col];
+            } else if (my_slot < n) {
+                have = true;
+                fl = k.flags[my_slot];
+                my_cell = k.idx[my_slot];
+                if (!kClassic) my_temp = k.ltemp[my_slot];
+                my_col = column(my_cell);
+                s.flags[tid] = (uint8_t)fl;
+                if ((fl & (kFrontIdle | kFrontQuiet | kFrontDead)) == kFrontIdle) seen = k.stamp[my_col];
+            }
+            if (have) {
+                const bool vent = (fl & kFrontVent) != 0;
+                if (fl & kFrontDead) {
+                    if (!kClassic && !(fl & kFrontStored)) {  // its last temperature, now that no vote reads it
+                        int x, y, z;
+                        front_decode(k, my_cell, x, y, z);
+                        k.temp[pidx(k.g, x, y, z)] = my_temp;
+                        s.flags[tid] = (uint8_t)(fl | kFrontStored);
+                    }
+                } else {
+                    if (kClassic) {
+                        ++my_active;
+                    } else {
+                        if (my_slot < prev) my_temp = front_cool(k, my_temp, vent, (int64_t)t - 1);  // the update of the last step
+                        const float next = front_cool(k, my_temp, vent, t);
+                        dying = next < k.solidus;
+                        if (dying) {
+                            ++my_changed;
+                            s.nsolid = 1;  // there is work for phase B
+                        } else {
+                            ++my_active;
+                            my_changed += next != my_temp;
+                        }
+                    }
+                    if (!(fl & kFrontQuiet) && seen == t - 1u) {  // an idle cell: the last step changed a type around its column
+                        const unsigned at = atomicAdd(&s.nqueue, 1u);  // kQueue >= kThreads
+                        s.q_slot[at] = (uint32_t)tid | (vent ? kVentBit : 0u);
+                        s.q_cell[at] = my_cell;
+                        s.q_temp[at] = my_temp;
+                    }
+                }
             }
             look();
         } else {
-            // four slots per thread, 8 threads per run; a full queue is emptied in between
-            for (uint32_t run0 = 0; run0 * nblk * 32u < n; run0 += 4 * (kThreads / 32)) {  // uniform over the block
-                const uint32_t base = ((run0 + 4 * warp + (lane >> 3)) * nblk + bid) * 32u + 4 * (lane & 7);
+            // four slots per thread, two threads per run; a full queue is emptied in between
+            for (uint32_t run0 = 0; run0 * nblk * kRun < n; run0 += 4 * kThreads / kRun) {  // uniform over the block
+                const uint32_t base = ((run0 + tid / 2) * nblk + bid) * kRun + 4 * (tid % 2);
                 unsigned want = 0;
                 uint32_t f4 = 0;
                 float te[4] = {0.f, 0.f, 0.f, 0.f};
                 uint32_t cell[4] = {0, 0, 0, 0};
                 if (base < n) {
                     f4 = *reinterpret_cast<const uint32_t*>(k.flags + base);
-                    if (!k.classic) {
+                    if (!kClassic) {
                         const float4 t4 = *reinterpret_cast<const float4*>(k.ltemp + base);
                         te[0] = t4.x, te[1] = t4.y, te[2] = t4.z, te[3] = t4.w;
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (base + j < n && cool(base + j, (f4 >> (8 * j)) & 0xFFu, te[j])) want |= 1u << j;
-                    if (!k.classic) *reinterpret_cast<float4*>(k.ltemp + base) = make_float4(te[0], te[1], te[2], te[3]);
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t slot = base + j;
+                        const unsigned fl = (f4 >> (8 * j)) & 0xFFu;
+                        if (slot >= n || (fl & kFrontDead)) continue;
+                        if (kClassic) {
+                            ++my_active;
+                        } else {
+                            const bool vent = (fl & kFrontVent) != 0;
+                            if (slot < prev) te[j] = front_cool(k, te[j], vent, (int64_t)t - 1);
+                            const float next = front_cool(k, te[j], vent, t);
+                            if (next < k.solidus) {
+                                ++my_changed;
+                                const unsigned at = atomicAdd(&s.nsolid, 1u);
+                                if (at < (unsigned)S::kSolid) s.solid[at] = slot;
+                                else k.work[k.work_cap - 1u - atomicAdd(&over[1], 1u)] = slot;
+                            } else {
+                                ++my_active;
+                                my_changed += next != te[j];
+                            }
+                        }
+                        if (!(fl & kFrontQuiet)) want |= 1u << j;
+                    }
+                    if (!kClassic) *reinterpret_cast<float4*>(k.ltemp + base) = make_float4(te[0], te[1], te[2], te[3]);
                     if (want) {
                         const uint4 c4 = *reinterpret_cast<const uint4*>(k.idx + base);
                         cell[0] = c4.x, cell[1] = c4.y, cell[2] = c4.z, cell[3] = c4.w;
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            if (((want >> j) & 1u) && ((f4 >> (8 * j)) & kFrontIdle) && !stale(cell[j])) want &= ~(1u << j);
+                            if (((want >> j) & 1u) && ((f4 >> (8 * j)) & kFrontIdle) && k.stamp[column(cell[j])] != t - 1u)
+                                want &= ~(1u << j);
                     }
                 }
                 for (;;) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (((want >> j) & 1u) && push(base + j, (f4 >> (8 * j)) & 0xFFu, cell[j], te[j])) want &= ~(1u << j);
+                    for (int j = 0; j < 4; ++j) {
+                        if (!((want >> j) & 1u)) continue;
+                        const unsigned at = atomicAdd(&s.nqueue, 1u);
+                        if (at >= (unsigned)S::kQueue) continue;
+                        s.q_slot[at] = (base + j) | ((f4 >> (8 * j)) & kFrontVent ? kVentBit : 0u);
+                        s.q_cell[at] = cell[j];
+                        s.q_temp[at] = te[j];
+                        want &= ~(1u << j);
+                    }
                     if (!__syncthreads_or(want != 0)) break;
                     look();
                     __syncthreads();
@@ -448,24 +577,24 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
         }
         __syncthreads();
         // ---- barrier: blocks with work for phase B, with active and with changed cells, with overflow lists
-        if (tid == 0) {
+        unsigned long long wordA = 0;
+        if (nblk == 1 || tid == 0) {
             const bool work = (s.ncand | s.nsolid) != 0, more = s.ncand > (unsigned)S::kCand || s.nsolid > (unsigned)S::kSolid;
-            const unsigned long long add = 1ull | ((unsigned long long)work << kWordBits) |
-                                           ((unsigned long long)(s.active != 0) << 2 * kWordBits) |
-                                           ((unsigned long long)(s.changed != 0) << 3 * kWordBits) |
-                                           ((unsigned long long)more << 4 * kWordBits);
-            s.word = front_arrive(ctrl, &ctrl->front_word[t % 3u][0], add, nblk);
-            s.nqueue = 0;
-        } else if (tid == 32) {
+            wordA = 1ull | ((unsigned long long)work << kWordBits) | ((unsigned long long)(s.active != 0) << 2 * kWordBits) |
+                    ((unsigned long long)(s.changed != 0) << 3 * kWordBits) | ((unsigned long long)more << 4 * kWordBits);
+            if (nblk > 1) s.word = front_arrive(ctrl, &ctrl->front_word[t % 3u][0], wordA, nblk);
+        }
+        if (tid == 32) {
             if (s.active) atomicAdd(&k.hist_active[t], (unsigned long long)s.active);
             if (s.changed) atomicAdd(&k.hist_changed[t], (unsigned long long)s.changed);
         }
         __syncthreads();
-        const unsigned long long wordA = s.word;
+        if (nblk > 1) wordA = s.word;
         if (wordA == 0ull) {
             ok = false;
             break;
         }
+        if (tid == 0) s.nqueue = s.active = s.changed = 0;  // used again after another __syncthreads
         if (bid == 0 && tid == 64) {  // step t + 2 starts at zero (its words' last readers passed the barrier above)
             const uint32_t r = (t + 2u) % 3u;
             ctrl->front_word[r][0] = ctrl->front_word[r][1] = 0ull;
@@ -476,111 +605,155 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
         if (field(1)) {
             // ---- phase B
             const uint16_t stamp = (uint16_t)min(t, 65535u);
-            auto note = [&](uint32_t c) {  // a cell whose type changed (its columns are stamped below)
-                const unsigned at = atomicAdd(&s.nqueue, 1u);
-                if (at < (unsigned)S::kQueue) s.q_cell[at] = c;
-                else
-                    for (int i = 0; i < 9; ++i) front_stamp(k, c, i, t);
+            // births in the lower half of the queue's arrays, hard votes in the upper one
+            auto birth = [&](uint32_t c, int x, int y, int z, int64_t p, int32_t nf, float nt) {
+                k.type[p] = kLava;
+                k.flow[p] = nf;
+                k.temp[p] = nt;
+                k.solid[p] = 0;
+                k.arrival[p] = stamp;
+                const bool vent = !kClassic && front_is_vent(k, nf, x, y, z);
+                const unsigned at = atomicAdd(&s.born, 1u);
+                if (at < (unsigned)kThreads) {
+                    s.q_slot[at] = vent ? kVentBit : 0u;
+                    s.q_cell[at] = c;
+                    s.q_temp[at] = nt;
+                } else {
+                    const unsigned slot = atomicAdd(&ctrl->front_n, 1u);
+                    k.idx[slot] = c;
+                    k.ltemp[slot] = nt;
+                    k.flags[slot] = vent ? kFrontVent : 0;
+                    stamp_type(c);
+                }
             };
             auto candidates = [&](uint32_t first, uint32_t count, uint32_t stride, const uint32_t* list) {
                 for (uint32_t base = first; base < count; base += stride) {  // uniform over the block
-                    const uint32_t j = base + tid;
-                    bool gained = false;
-                    uint32_t c = 0;
-                    int x = 0, y = 0, z = 0;
-                    int64_t p = 0;
-                    int32_t nf = 0;
-                    float nt = 0.f;
-                    if (j < count) {
-                        c = list[j];
+                    uint32_t hard = 0;
+                    if (base + tid < count) {
+                        const uint32_t c = list[base + tid];
+                        int x, y, z;
                         front_decode(k, c, x, y, z);
-                        p = pidx(k.g, x, y, z);
-                        gained = front_decide(k, c, x, y, z, p, t, nf, nt);
+                        const int64_t p = pidx(k.g, x, y, z);
+                        int32_t nf = 0;
+                        float nt = 0.f;
+                        if (front_decide<kClassic>(k, c, x, y, z, p, t, nf, nt, hard)) birth(c, x, y, z, p, nf, nt);
+                        if (hard) {
+                            const unsigned at = kThreads + atomicAdd(&s.nqueue, 1u);
+                            s.q_slot[at] = hard;
+                            s.q_cell[at] = c;
+                        }
                     }
-                    const unsigned who = __ballot_sync(0xFFFFFFFFu, gained);
-                    if (!who) continue;
-                    unsigned at = 0;
-                    if (lane == 0) {
-                        at = atomicAdd(&ctrl->front_n, (unsigned)__popc(who));
-                        atomicAdd(&s.born, (unsigned)__popc(who));
+                    if (!__syncthreads_or(hard != 0)) continue;
+                    const unsigned nh = s.nqueue;
+                    for (unsigned j = warp; j < nh; j += kThreads / 32) {
+                        const uint32_t c = s.q_cell[kThreads + j];
+                        int32_t nf;
+                        float nt;
+                        front_vote<kClassic>(k, c, s.q_slot[kThreads + j], t, lane, nf, nt);
+                        if (lane == 0 && (kClassic || nt >= k.solidus)) {
+                            int x, y, z;
+                            front_decode(k, c, x, y, z);
+                            birth(c, x, y, z, pidx(k.g, x, y, z), nf, nt);
+                        }
                     }
-                    if (gained) {
-                        k.type[p] = kLava;
-                        k.flow[p] = nf;
-                        k.temp[p] = nt;
-                        k.solid[p] = 0;
-                        k.arrival[p] = stamp;
-                        note(c);
-                    }
-                    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(who & ((1u << lane) - 1u));
-                    if (gained) {
-                        k.idx[at] = c;
-                        k.ltemp[at] = nt;
-                        k.flags[at] = front_is_vent(k, nf, x, y, z) ? kFrontVent : 0;
-                    }
+                    __syncthreads();
+                    if (tid == 0) s.nqueue = 0;
+                    __syncthreads();
                 }
             };
-            auto solidify = [&](uint32_t slot) {
-                const uint32_t c = k.idx[slot];
+            // A dead cell's temperature does not go into the plane yet: as a source of this step's votes the
+            // cell still has the one before.
+            auto solidify = [&](uint32_t c) {
                 int x, y, z;
                 front_decode(k, c, x, y, z);
                 const int64_t p = pidx(k.g, x, y, z);
                 k.type[p] = kBasalt;
                 k.solid[p] = stamp;
-                // not into the plane: as a source of this step's votes the cell still has the temperature before
+                stamp_type(c);
+            };
+            auto solidify_slot = [&](uint32_t slot) {
                 k.ltemp[slot] = front_cool(k, k.ltemp[slot], (k.flags[slot] & kFrontVent) != 0, t);
                 k.flags[slot] = kFrontDead;
-                note(c);
+                solidify(k.idx[slot]);
             };
-            const uint32_t nc = min(s.ncand, (unsigned)S::kCand), ns = min(s.nsolid, (unsigned)S::kSolid);
-            candidates(0, nc, kThreads, s.cand);
-            for (uint32_t j = tid; j < ns; j += kThreads) solidify(s.solid[j]);
+            __syncthreads();  // the queue counters are clear
+            candidates(0, min(s.ncand, (unsigned)S::kCand), kThreads, s.cand);
+            if (resident) {
+                if (dying) {
+                    my_temp = front_cool(k, my_temp, (s.flags[tid] & kFrontVent) != 0, t);
+                    s.flags[tid] = kFrontDead;
+                    dying = false;
+                    solidify(my_cell);
+                }
+            } else {
+                const uint32_t ns = min(s.nsolid, (unsigned)S::kSolid);
+                for (uint32_t j = tid; j < ns; j += kThreads) solidify_slot(s.solid[j]);
+            }
             if (field(4)) {  // overflow lists, shared by all blocks
                 const uint32_t oc = __ldcg(&over[0]), os = __ldcg(&over[1]);
                 candidates(bid * kThreads, oc, T, k.work);
-                for (uint32_t j = bid * kThreads + tid; j < os; j += T) solidify(__ldcg(k.work + (k.work_cap - 1u - j)));
+                for (uint32_t j = bid * kThreads + tid; j < os; j += T) solidify_slot(__ldcg(k.work + (k.work_cap - 1u - j)));
             }
             __syncthreads();
-            const unsigned nt = 9u * min(s.nqueue, (unsigned)S::kQueue);
-            for (unsigned j = tid; j < nt; j += kThreads) front_stamp(k, s.q_cell[j / 9u], j % 9u, t);
-            __syncthreads();
+            // the block's births: their place in the list, meanwhile the stamps around them
+            const unsigned nb = s.born, listed = min(nb, (unsigned)kThreads);
+            if (listed) {
+                if (tid == 0) s.base = atomicAdd(&ctrl->front_n, listed);
+                for (unsigned j = tid; j < 9u * listed; j += kThreads) front_stamp(k, s.q_cell[j / 9u], j % 9u, t);
+                __syncthreads();
+                for (unsigned j = tid; j < listed; j += kThreads) {
+                    const unsigned slot = s.base + j;
+                    k.idx[slot] = s.q_cell[j];
+                    k.ltemp[slot] = s.q_temp[j];
+                    k.flags[slot] = s.q_slot[j] ? kFrontVent : 0;
+                }
+                __syncthreads();
+            }
+            unsigned long long wordB = 1ull | ((unsigned long long)nb << kWordBits);
             if (tid == 0) {
-                s.word = front_arrive(ctrl, &ctrl->front_word[t % 3u][1], 1ull | ((unsigned long long)s.born << kWordBits), nblk);
-                s.nqueue = s.ncand = s.nsolid = 0;
-            } else if (tid == 32 && s.born) {
-                atomicAdd(&k.hist_active[t], (unsigned long long)s.born);
-                atomicAdd(&k.hist_changed[t], (unsigned long long)s.born);
+                if (nblk > 1) s.word = front_arrive(ctrl, &ctrl->front_word[t % 3u][1], wordB, nblk);
+                s.ncand = s.nsolid = 0;
+            } else if (tid == 32 && nb) {
+                atomicAdd(&k.hist_active[t], (unsigned long long)nb);
+                atomicAdd(&k.hist_changed[t], (unsigned long long)nb);
             }
             __syncthreads();
-            if (s.word == 0ull) {
+            if (nblk > 1) wordB = s.word;
+            if (wordB == 0ull) {
                 ok = false;
                 break;
             }
-            born = (uint32_t)(s.word >> kWordBits);
+            if (tid == 0) s.born = 0;
+            born = (uint32_t)(wordB >> kWordBits);
         }
-        if (tid == 0) s.active = s.changed = s.born = 0;  // used again after the next __syncthreads
         // ---- finishStep (LavaCA.hpp:1206-1229), the same in every block
         air -= born;
         visited += n;
         prev = n;
         n += born;
         ++t;
-        if (!k.classic && !field(2) && !born) stop = VCA_STOP_NO_LAVA;
-        else if (k.classic && air == 0) stop = VCA_STOP_NO_AIR;
+        if (!kClassic && !field(2) && !born) stop = VCA_STOP_NO_LAVA;
+        else if (kClassic && air == 0) stop = VCA_STOP_NO_AIR;
         else if (!field(3) && !born && !k.random_nb) stop = VCA_STOP_NO_CHANGE;
         else if ((int)t >= k.max_steps) stop = VCA_STOP_MAX_STEPS;
+        if (!field(1)) __syncthreads();  // the counters are clear before the next phase A
     }
-    if (ok && !k.classic) {
+    if (ok && resident) write_back();
+    if (ok && !kClassic) {
         // the temperatures of the LAVA cells back into their plane, and once those of the dead ones
-        for (uint32_t slot = bid * kThreads + tid; slot < n; slot += T) {
-            const uint8_t fl = k.flags[slot];
-            if (fl & kFrontStored) continue;
-            float te = k.ltemp[slot];
-            if (fl & kFrontDead) k.flags[slot] = fl | kFrontStored;
+        auto store = [&](uint32_t slot, unsigned fl, uint32_t cell, float te) {
+            if (fl & kFrontStored) return;
+            if (fl & kFrontDead) k.flags[slot] = (uint8_t)(fl | kFrontStored);
             else if (slot < prev) te = front_cool(k, te, (fl & kFrontVent) != 0, (int64_t)t - 1);
             int x, y, z;
-            front_decode(k, k.idx[slot], x, y, z);
+            front_decode(k, cell, x, y, z);
             k.temp[pidx(k.g, x, y, z)] = te;
+        };
+        if (resident) {
+            // (a slot born in the last step is not resident yet; its plane has its temperature)
+            if (have) store(my_slot, s.flags[tid], my_cell, my_temp);
+        } else {
+            for (uint32_t slot = bid * kThreads + tid; slot < n; slot += T) store(slot, k.flags[slot], k.idx[slot], k.ltemp[slot]);
         }
     }
     __syncthreads();
@@ -609,10 +782,11 @@ __device__ __forceinline__ void front_body(const CaFrontArgs& k, FrontShared<kTh
     for (int i = lane; i < (int)(sizeof(CaCtrl) / sizeof(uint32_t)); i += 32) to[i] = __ldcg(from + i);
 }
 
-__global__ __launch_bounds__(kFrontThreads, 1) void ca_front_kernel(const __grid_constant__ CaFrontArgs k, int steps,
-                                                                    uint32_t most, CaCtrl* snap) {
-    __shared__ FrontShared<kFrontThreads> s;
-    front_body<kFrontThreads>(k, s, blockIdx.x, gridDim.x, steps, most, snap);
+template <int kThreads, bool kClassic>
+__global__ __launch_bounds__(kThreads, 1) void ca_front_kernel(const __grid_constant__ CaFrontArgs k, int steps, uint32_t most,
+                                                               CaCtrl* snap) {
+    __shared__ FrontShared<kThreads> s;
+    front_body<kThreads, kClassic>(k, s, blockIdx.x, gridDim.x, steps, most, snap);
 }
 
 // Many grids in one launch: a block serves one member, `n[slot]` blocks share a member's steps and its
@@ -627,7 +801,8 @@ __global__ __launch_bounds__(kFrontBatchThreads, 4) void ca_front_batch_kernel(c
     for (int i = threadIdx.x; i < (int)(sizeof(CaFrontArgs) / sizeof(uint2)); i += blockDim.x)
         reinterpret_cast<uint2*>(&s_k)[i] = from[i];
     __syncthreads();
-    front_body<kFrontBatchThreads>(s_k, s, (uint32_t)m.y, (uint32_t)b.n[m.x], steps, 0xFFFFFFFFu, nullptr);
+    if (s_k.classic) front_body<kFrontBatchThreads, true>(s_k, s, (uint32_t)m.y, (uint32_t)b.n[m.x], steps, 0xFFFFFFFFu, nullptr);
+    else front_body<kFrontBatchThreads, false>(s_k, s, (uint32_t)m.y, (uint32_t)b.n[m.x], steps, 0xFFFFFFFFu, nullptr);
 }
 
 // The front list of the current planes: every LAVA cell, 16 cells of a row per thread (a row is a
@@ -767,9 +942,24 @@ cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cu
 }
 
 constexpr int kFrontChunk = 64;        // steps per launch of a run
-// Slots up to which one block steps the grid: its step has no grid barriers, but a few hundred cells that
-// look around at once keep its 32 warps busy for longer than the barriers of all SMs cost.
-constexpr uint32_t kFrontSolo = 2048;
+
+// The launch for a list of n slots.  Up to kFrontSolo one small block: its step has no grid barrier and each
+// of its barriers waits for 8 warps only (512 x 1 x 256, 300 steps: 1.54 ms; left to all SMs above 256 slots
+// 1.84 ms; one block of 1024 threads 1.9 ms).  Up to kFrontSmall blocks of 256 threads on all SMs, which hold
+// a slot per thread in registers up to 37 888 slots; beyond, the list is streamed and 1024 threads stream it
+// faster (256 x 256 x 128, 400 steps: 2.80 ms with the line at 40 000, 2.98 ms without the small blocks;
+// classic 100^3: 1.21 ms, with the line at 160 000 1.34 ms).  A launch ends early when its list has
+// outgrown `most`.
+constexpr uint32_t kFrontSolo = 512, kFrontSmall = 40000;
+struct FrontShape {
+    int threads, blocks;
+    uint32_t most;
+};
+static FrontShape front_shape(const vca_ca* h, uint64_t n) {
+    if (n <= kFrontSolo) return {256, 1, kFrontSolo};
+    if (n <= kFrontSmall) return {256, h->sms, 2 * kFrontSmall};
+    return {kFrontThreads, h->sms, 0xFFFFFFFFu};
+}
 
 vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
     if (!h->front_listed)
@@ -778,16 +968,18 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
     VCA_CUDA(cudaEventRecord(h->ev_a, h->stream));
     CaCtrl last = *h->ctrl_host;
     auto launch = [&](int steps, uint32_t n, int slot) -> vca_status {
-        // one block while the list is short (it leaves the launch when it has outgrown it), else all SMs
-        const bool solo = n <= kFrontSolo;
-        uint32_t most = solo && until_stop ? kFrontSolo : 0xFFFFFFFFu;
+        const FrontShape f = front_shape(h, n);
+        uint32_t most = until_stop ? f.most : 0xFFFFFFFFu;
         CaCtrl* snap = h->ctrl_ring_dev + slot;
-        if (solo) {
-            ca_front_kernel<<<1, kFrontThreads, 0, h->stream>>>(k, steps, most, snap);
+        const bool small = f.threads == 256;
+        const auto kernel = small ? (k.classic ? ca_front_kernel<256, true> : ca_front_kernel<256, false>)
+                                  : (k.classic ? ca_front_kernel<kFrontThreads, true> : ca_front_kernel<kFrontThreads, false>);
+        if (f.blocks == 1) {
+            kernel<<<1, f.threads, 0, h->stream>>>(k, steps, most, snap);
             VCA_CUDA(cudaGetLastError());
         } else {
             void* args[] = {&k, &steps, &most, &snap};
-            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)ca_front_kernel, h->sms, kFrontThreads, args, 0, h->stream));
+            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, f.blocks, f.threads, args, 0, h->stream));
         }
         h->launches += 1;
         return VCA_OK;
