@@ -61,3 +61,39 @@ def test_space_sweeps_match_oracle(case):
     info = mc.info()
     assert (info.attempts, info.accepted, info.uphill, info.sweeps) == (*(int(v) for v in tot), done)
     mc.close()
+
+
+@pytest.mark.parametrize("case", [("moore", "periodic", (6, 5, 4), 20, 0.7, False), ("moore", "periodic", (17, 9, 7), 256, 0.5, True),
+                                  ("von_neumann", "periodic", (17, 9, 4), 64, 0.5, True), ("pentagonal", "absorbing", (40, 9, 6), 129, 0.6, True),
+                                  ("hexagonal", "periodic", (31, 17, 1), 2, 0.0, False), ("von_neumann", "absorbing", (480, 200, 1), 9, 0.5, False),
+                                  ("von_neumann", "absorbing", (480, 201, 1), 9, 0.5, False)],
+                         ids=lambda c: f"{c[0]}-{c[1]}-{'x'.join(map(str, c[2]))}-Q{c[3]}")
+def test_small_spaces_match_oracle(case):
+    """Calls of four and more MCS on small spaces (a cell per thread) and shorter calls before and after them,
+    up to the widest colour that is still taken that way and one row beyond."""
+    nb, bc, (nx, ny, nz), Q, kT, use_mob = case
+    seed = 31 + nx + 3 * ny
+    n = nx * ny * nz
+    domain = np.ones(n, np.uint8)
+    mob = np.random.default_rng(seed).uniform(0.2, 1.0, n).astype(np.float32) if use_mob else None
+    mp = O.mc_params(nx, ny, nz, nb, bc, True, seed, Q, 1.0, kT)
+    spin = O.mc_init(mp, domain)
+    mc = capi.PottsMC(capi.McParams(nx, ny, nz, neighborhood=nb, boundary=bc, domain_full=True, seed=seed, Q=Q, kT=kT))
+    mc.set_domain(None)
+    if use_mob:
+        mc.set_mobility(mob)
+    mc.initialize()
+    tot = np.zeros(3, np.uint64)
+    done = 0
+    for count in (1, 4, 2, 5):
+        before = int(tot[1])
+        for _ in range(count):
+            tot += O.mc_sweep(mp, done, domain, mob, spin)
+            done += 1
+        assert mc.sweep(count) == int(tot[1]) - before
+        got = mc.crystals()
+        assert np.array_equal(got, spin), f"sweep {done}: {(got != spin).sum()} cells differ"
+        assert mc.energy() == O.mc_energy(mp, done, spin)
+    info = mc.info()
+    assert (info.attempts, info.accepted, info.uphill, info.sweeps) == (*(int(v) for v in tot), done)
+    mc.close()

@@ -643,7 +643,7 @@ __global__ __launch_bounds__(kMcThreads, 2) void mc_sweeps_kernel(const __grid_c
 // What bounds it: the integer ALU (79 % busy), three 64-bit hashes of a trial (two at kT = 0) above all.
 // Per MCS on one B200 against a thread per cell with 26 byte loads and compares (709 instructions per
 // trial): 512 x 512 x 256 Moore, Q = 64, kT = 0.5 1.80 -> 0.79 ms, the same von Neumann 1.88 -> 0.54 ms,
-// 256 x 256 x 128 pentagonal 0.30 -> 0.16 ms, 50^3 Moore 38 -> 29 us.  Three resident blocks per SM
+// 256 x 256 x 128 pentagonal 0.30 -> 0.16 ms, 100^3 Moore 38 -> 31 us.  Three resident blocks per SM
 // instead of two (80 registers, spills) 0.85 ms; moving adds and shifts to the FMA pipe 0.89 ms.
 // ------------------------------------------------------------------------------------------
 constexpr int kSpaceBlocks = 2;  // resident blocks per SM the registers are limited to
@@ -1346,8 +1346,8 @@ __device__ __forceinline__ void gr_union(uint32_t* parent, uint32_t a, uint32_t 
 // over the forward offsets of the connectivity (dz, dy, dx order) on the axes of size > 1; sizes and high
 // cells per root; the statistics, summed per block before they reach the counters.  The last block hands
 // them to the host (out: host-mapped).  With a few 10^5 cells the four passes are latencies; separate
-// launches with an atomic per thread and counter took 2.05 ms for 401 K cells and 0.18 ms for 50^3, this
-// one GRAIN_NOW.
+// launches with an atomic per thread and counter took 2.05 ms a call for 401 K cells and 0.18 ms for 50^3,
+// this one 0.10 and 0.07 ms.
 __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_constant__ McArgs a, const uint32_t* list,
                                                                uint64_t count, int moore, const float* mob, double threshold,
                                                                uint32_t* parent, uint32_t* gsize, uint32_t* ghigh, GrainAcc* acc,
@@ -1878,6 +1878,22 @@ bool space_applies(const vca_mc* h) {
            h->color_off.back() == h->n && h->n > 0 && nx >= 6;
 }
 
+// A whole space whose colours leave a thread of the grid about one cell: the listed kernel's pass, a cell
+// per thread and its draws done while the block waits, is then shorter than four cells per thread.  Per MCS
+// of 8 colours, listed against four cells: 50^3 18 / 31 us, 64^3 21 / 30, 80^3 (64 000 cells a colour)
+// 26 / 30 and level with the lists' set-up in calls of 5 MCS, 100^3 32 / 31; 512 x 512 in 4 colours of
+// 65 536 12.5 / 15.4.  The lists cost what four MCS save; a handle made for a much larger space would
+// allocate them for it.
+constexpr uint64_t kListWhole = 48000;   // cells of the widest colour
+constexpr int kListWholeSweeps = 4;
+bool small_space_listed(const vca_mc* h, int count) {
+    if (h->user_spins || h->desc.Q > 256 || h->desc.nx < 6 || h->slab_zoff >= 0) return false;
+    if (!h->listed && (count < kListWholeSweeps || (!h->list && h->cap_n > 64 * kListWhole))) return false;
+    uint64_t widest = 0;
+    for (int c = 0; c < h->colors; ++c) widest = std::max<uint64_t>(widest, h->color_off[c + 1] - h->color_off[c]);
+    return widest <= kListWhole;
+}
+
 // The byte copy's shape and the colour classes; `a` becomes the sweep's view of a turned space.
 McSpace space_args(const vca_mc* h, McArgs& a) {
     McSpace d;
@@ -2287,7 +2303,7 @@ vca_status vca_mc_sweep(vca_mc* h, int count, uint64_t* accepted) {
     };
     if (!h->profile_kernels) {
         // all sweeps in one cooperative launch (colour passes separated by grid barriers)
-        const bool space = space_applies(h);
+        const bool space = space_applies(h) && !small_space_listed(h, count);
         VCA_CUDA(cudaEventRecord(h->ev_a, h->stream));
         if (count > 0 && space) {
             // whole space: sweeps on the byte copy of the orientations, copied back after
@@ -2472,7 +2488,7 @@ vca_status vca_mc_grains(vca_mc* h, int moore, double mobility_threshold, vca_mc
         VCA_CUDA(cudaMemsetAsync(acc, 0, sizeof(GrainAcc), h->stream));
         VCA_CUDA(cudaMemsetAsync(&h->ctrl->bar_arrived, 0, sizeof(unsigned long long), h->stream));
         const int grid = (int)std::min<uint64_t>((total + kMcThreads - 1) / kMcThreads, (uint64_t)h->sms * h->grain_per_sm);
-        const uint32_t* list = h->listed ? h->list : nullptr;  // none: every cell in order
+        const uint32_t* list = total < h->n ? h->list : nullptr;  // none: every cell in order (also where there is a list)
         volatile GrainAcc* out = h->gacc_host_dev;
         void* args[] = {&a, &list, &total, &moore, &mob, &mobility_threshold, &h->gparent, &h->gsize, &h->ghigh, &acc, &out};
         VCA_CUDA(cudaLaunchCooperativeKernel((const void*)mc_grains_kernel, grid, kMcThreads, args, 0, h->stream));
@@ -2517,7 +2533,7 @@ vca_status vca_mc_energy(vca_mc* h, double* energy) {
     VCA_CUDA(cudaMemsetAsync(&h->ctrl->energy_acc, 0, 8, h->stream));
     const uint64_t total = h->color_off.back();
     const bool forward = h->nb_host.variants == 1;
-    if (total) mc_energy_kernel<<<grid_for(total, h->sms), kMcThreads, 0, h->stream>>>(mc_args(h), h->listed ? h->list : nullptr, total, forward);
+    if (total) mc_energy_kernel<<<grid_for(total, h->sms), kMcThreads, 0, h->stream>>>(mc_args(h), total < h->n ? h->list : nullptr, total, forward);
     h->launches += total ? 1 : 0;
     VCA_CUDA(cudaGetLastError());
     if (vca_status s_ = mc_sync(h)) return s_;
