@@ -71,3 +71,32 @@ def test_grain_statistics_match_connected_components(case):
                g.low_grain_cells, g.low_largest)
         assert got == _host(spins, dims, nb == "moore", bc == "periodic", mob, 0.5)
     mc.close()
+
+
+@pytest.mark.parametrize("listed", [False, True], ids=["whole", "partial"])
+@pytest.mark.parametrize("nb", ["moore", "von_neumann"])
+@pytest.mark.parametrize("dims", [(33, 6, 5), (64, 5, 4), (2, 3, 5), (3, 2, 2), (1, 7, 9), (100, 2, 1)], ids=lambda d: "x".join(map(str, d)))
+def test_grains_of_whole_rows(dims, nb, listed):
+    """Runs as long as their row, rings on a periodic axis, pairs of rows that only their ends join, axes of
+    one to three cells."""
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nx + 7 * ny)
+    z, y, x = np.meshgrid(np.arange(nz), np.arange(ny), np.arange(nx), indexing="ij")
+    for periodic in (True, False):
+        for k, spins in enumerate((1 + y // 2 % 2 + 2 * (z % 2), 1 + (x + y) // 3 % 2, np.where(x == nx - 1, 1, 2 + (y + z) % 2),
+                                   rng.integers(1, 3, (nz, ny, nx)))):
+            spins = spins.astype(np.int32).reshape(-1)
+            domain = np.ones(spins.size, np.uint8)
+            if listed:
+                domain[rng.integers(0, spins.size, max(1, spins.size // 9))] = 0
+                spins = spins * domain
+            mc = capi.PottsMC(capi.McParams(*dims, neighborhood=nb, boundary="periodic" if periodic else "absorbing", domain_full=True,
+                                            seed=1, Q=64))
+            mc.set_domain(domain)
+            mc.initialize()
+            mc.set_spins(spins)
+            g = mc.grains(moore=nb == "moore", threshold=0.5)
+            got = (g.grains, g.cells, g.largest, g.high_cells, g.high_grains, g.high_grain_cells, g.high_largest, g.low_grains,
+                   g.low_grain_cells, g.low_largest)
+            assert got == _host(spins, dims, nb == "moore", periodic, None, 0.5), (periodic, k)
+            mc.close()

@@ -1295,12 +1295,18 @@ __global__ __launch_bounds__(kListThreads, 1) void mc_list_sweeps_kernel(const _
 
 // PottsMC::totalEnergy (PottsMC.cpp:590-664): unlike pairs.  Deterministic neighbourhoods count
 // each pair once through the forward offsets; random ones sum E_i over the cells with the
-// variant of MCS t (the caller halves it).
-__global__ __launch_bounds__(kMcThreads) void mc_energy_kernel(McArgs a, const uint32_t* list, uint64_t count, int forward) {
+// variant of MCS t (the caller halves it).  Bounded by the launch and the wait for it: the neighbours of a
+// cell are loaded together.  One after another through the neighbourhood's table a call for 50^3 Moore took
+// 24 us, for 401 K listed pentagonal cells 47; now 18 and 31.
+struct McMasks {
+    uint32_t of[6];  // per variant: bit (dx + 1) + 3 (dy + 1) + 9 (dz + 1) of each neighbour
+};
+template <bool kForward>
+__global__ __launch_bounds__(kMcThreads) void mc_energy_kernel(const __grid_constant__ McArgs a, const __grid_constant__ McMasks m,
+                                                               const uint32_t* list, uint64_t count) {
     __shared__ unsigned long long s_sum;
     if (threadIdx.x == 0) s_sum = 0;
     __syncthreads();
-    const NbTable& nb = *a.nb;
     const uint64_t prefix = hash_prefix(a.seed, a.ctrl->sweeps);
     unsigned long long mine = 0;
     for (uint64_t j = blockIdx.x * (uint64_t)kMcThreads + threadIdx.x; j < count; j += (uint64_t)gridDim.x * kMcThreads) {
@@ -1309,17 +1315,28 @@ __global__ __launch_bounds__(kMcThreads) void mc_energy_kernel(McArgs a, const u
         decode(a, g, x, y, z);
         const int32_t s = a.spin[g];
         int var = 0;
-        if (!forward && a.variants > 1)
+        if (!kForward && a.variants > 1)
             var = (int)fast_mod(hash_salt(hash_index(prefix, g + a.gidx_base), kSaltNeighborhood), a.var_mod);
-        int in_dom = 0, same = 0;
-        for (int k = 0; k < nb.count[var]; ++k) {
-            const int dx = nb.off[var][k][0], dy = nb.off[var][k][1], dz = nb.off[var][k][2];
-            if (forward && !(dz > 0 || (dz == 0 && (dy > 0 || (dy == 0 && dx > 0))))) continue;
-            const int32_t sj = spin_at(a, x + dx, y + dy, z + dz);
-            in_dom += sj != 0;
-            same += sj == s;
+        const uint32_t mask = m.of[var];
+        int64_t ox[3], oy[3], oz[3];
+        bool kx[3], ky[3], kz[3];
+        mc_axis_nb(x, a.nx, a.per[0], 1, ox, kx);
+        mc_axis_nb(y, a.ny, a.per[1], a.nx, oy, ky);
+        mc_axis_nb(z, a.nz, a.per[2], (int64_t)a.nx * a.ny, oz, kz);
+        const uint32_t dx[3] = {(uint32_t)ox[0], 0u, (uint32_t)ox[2]}, dy[3] = {(uint32_t)oy[0], 0u, (uint32_t)oy[2]},
+                       dz[3] = {(uint32_t)oz[0], 0u, (uint32_t)oz[2]};  // (below 2^32 cells)
+        int32_t v[27];
+#pragma unroll
+        for (int i = kForward ? 14 : 0; i < 27; ++i) {
+            v[i] = 0;
+            if (i != 13 && ((mask >> i) & 1u) && kx[i % 3] && ky[i / 3 % 3] && kz[i / 9])
+                v[i] = a.spin[g + dx[i % 3] + dy[i / 3 % 3] + dz[i / 9]];
         }
-        mine += (unsigned long long)(in_dom - same);
+        int unlike = 0;
+#pragma unroll
+        for (int i = kForward ? 14 : 0; i < 27; ++i)
+            if (i != 13 && ((mask >> i) & 1u)) unlike += (int)(v[i] != 0) - (int)(v[i] == s);
+        mine += (unsigned long long)unlike;
     }
     for (int off = 16; off > 0; off >>= 1) mine += __shfl_down_sync(0xFFFFFFFFu, mine, off);
     if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, mine);
@@ -1373,23 +1390,41 @@ __device__ __forceinline__ void gr_union(uint32_t* parent, uint32_t a, uint32_t 
     atomicOr(err, 1u);
 }
 
-// All passes in one cooperative launch (a grid barrier after each): every cell its own grain; unions
+// All passes in one cooperative launch (a grid barrier after each): every cell under its run in x; unions
 // over the forward offsets of the connectivity (dz, dy, dx order) on the axes of size > 1; sizes and high
 // cells per root; the statistics, summed per block before they reach the counters.  The last block hands
 // them to the host (out: host-mapped).  With a few 10^5 cells the four passes are latencies; separate
 // launches with an atomic per thread and counter took 2.05 ms a call for 401 K cells and 0.18 ms for 50^3,
-// this one 0.10 and 0.07 ms.
+// this one 0.094 and 0.064 ms (0.039 before the first sweep: what is left grows with the unions).
 __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_constant__ McArgs a, const uint32_t* list,
                                                                uint64_t count, int moore, const float* mob, double threshold,
                                                                uint32_t* parent, uint32_t* gsize, uint32_t* ghigh, GrainAcc* acc,
                                                                GrainAcc* out) {
     const uint64_t i0 = blockIdx.x * (uint64_t)kMcThreads + threadIdx.x, T = (uint64_t)gridDim.x * kMcThreads;
     const int lane = threadIdx.x & 31;
-    for (uint64_t j = i0; j < count; j += T) {
-        const uint32_t g = list ? list[j] : (uint32_t)j;
-        parent[g] = g;
-        gsize[g] = 0;
-        ghigh[g] = 0;
+    // a cell starts under the first cell of its run of one orientation in x, as far as the warp (in cell
+    // order) or four cells (a list) show it; rows that wrap are united below
+    for (uint64_t base = i0 - lane; base < count; base += T) {  // uniform over the warp
+        const uint64_t j = base + lane;
+        const uint32_t g = j < count ? (list ? list[j] : (uint32_t)j) : 0u;
+        const uint32_t x = g % (uint32_t)a.nx;
+        const int32_t sg = a.spin[g];
+        uint32_t back = 0;
+        if (list) {
+            uint32_t same = 0;
+#pragma unroll
+            for (uint32_t i = 1; i <= 4; ++i) same |= (uint32_t)(x >= i && a.spin[x >= i ? g - i : g] == sg) << i;
+            while ((same >> (back + 1)) & 1u) ++back;
+        } else {
+            const bool on = x != 0 && a.spin[x != 0 ? g - 1u : g] == sg;
+            const unsigned heads = ~__ballot_sync(0xFFFFFFFFu, on) & (0xFFFFFFFFu >> (31 - lane));
+            back = heads ? lane - (31 - __clz(heads)) : lane + 1;
+        }
+        if (j < count) {
+            parent[g] = g - back;
+            gsize[g] = 0;
+            ghigh[g] = 0;
+        }
     }
     mc_barrier_arrive(a.ctrl);
     if (!mc_barrier_wait(a.ctrl, gridDim.x, 1)) return;
@@ -1399,25 +1434,41 @@ __global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_cons
         if (sg <= 0) continue;
         int x, y, z;
         decode(a, g, x, y, z);
-        // the neighbours of the same orientation first, all loads together, then their unions
+        // the forward neighbours and the left one, all loads together: bit i alike
+        int64_t ox[3], oy[3], oz[3];
+        bool kx[3], ky[3], kz[3];
+        mc_axis_nb(x, a.nx, a.per[0], 1, ox, kx);
+        mc_axis_nb(y, a.ny, a.per[1], a.nx, oy, ky);
+        mc_axis_nb(z, a.nz, a.per[2], (int64_t)a.nx * a.ny, oz, kz);
+        auto at = [&](int i) -> int64_t { return (int64_t)g + ox[i % 3] + oy[i / 3 % 3] + oz[i / 9]; };
         uint32_t alike = 0;
 #pragma unroll
-        for (int i = 14; i < 27; ++i) {  // the forward half of the 3 x 3 x 3 block
-            const int dx = i % 3 - 1, dy = i / 3 % 3 - 1, dz = i / 9 - 1;
-            int qx = x + dx, qy = y + dy, qz = z + dz;
-            bool in = !((a.nx == 1 && dx) || (a.ny == 1 && dy) || (a.nz == 1 && dz)) && (moore || abs(dx) + abs(dy) + abs(dz) == 1);
-            in = in && mc_wrap(qx, a.nx, a.per[0]) && mc_wrap(qy, a.ny, a.per[1]) && mc_wrap(qz, a.nz, a.per[2]);
-            const uint32_t q = in ? (uint32_t)qx + (uint32_t)a.nx * ((uint32_t)qy + (uint32_t)a.ny * (uint32_t)qz) : g;
-            const int32_t sq = a.spin[q];
-            alike |= (uint32_t)(in && sq == sg) << i;
+        for (int i = 12; i < 27; ++i) {
+            if (i == 13) continue;
+            const bool in = kx[i % 3] && ky[i / 3 % 3] && kz[i / 9];
+            const int32_t v = a.spin[in ? at(i) : (int64_t)g];
+            alike |= (uint32_t)(in && v == sg) << i;
         }
-        for (; alike; alike &= alike - 1) {
-            const int i = __ffs(alike) - 1;
-            int qx = x + i % 3 - 1, qy = y + i / 3 % 3 - 1, qz = z + i / 9 - 1;
-            mc_wrap(qx, a.nx, a.per[0]);
-            mc_wrap(qy, a.ny, a.per[1]);
-            mc_wrap(qz, a.nz, a.per[2]);
-            gr_union(parent, g, (uint32_t)qx + (uint32_t)a.nx * ((uint32_t)qy + (uint32_t)a.ny * (uint32_t)qz), &acc->error);
+        // of a row's three only the unions that no other cell's give: the row's cells hang together, and
+        // what the left (right) neighbour shares with the row it unites itself
+        // (the first cell of a row that wraps unites for itself, or a ring would leave it to nobody)
+        const bool left = ((alike >> 12) & 1u) && x > 0, right = (alike >> 14) & 1u;
+        uint32_t todo = right && x == a.nx - 1 ? 1u << 14 : 0u;
+#pragma unroll
+        for (int row = 5; row < 9; ++row) {
+            if (!moore && row != 5 && row != 7) continue;  // (y + 1, z) or (y, z + 1)
+            const uint32_t r = alike >> (3 * row);
+            const bool l = r & 1u, m = r & 2u, n = r & 4u;
+            if (m && !(left && l)) todo |= 2u << (3 * row);
+            if (moore && l && !m && !left) todo |= 1u << (3 * row);
+            if (moore && n && !m && !right) todo |= 4u << (3 * row);
+        }
+        for (; todo; todo &= todo - 1) {
+            const int i = __ffs(todo) - 1;
+            const int dx = i % 3, dy = i / 3 % 3, dz = i / 9;
+            const int64_t q = (int64_t)g + (dx == 0 ? ox[0] : dx == 2 ? ox[2] : 0) + (dy == 0 ? oy[0] : dy == 2 ? oy[2] : 0) +
+                              (dz == 2 ? oz[2] : 0);
+            gr_union(parent, g, (uint32_t)q, &acc->error);
         }
     }
     mc_barrier_arrive(a.ctrl);
@@ -2569,7 +2620,14 @@ vca_status vca_mc_energy(vca_mc* h, double* energy) {
     VCA_CUDA(cudaSetDevice(h->device));
     const uint64_t total = h->color_off.back();
     const bool forward = h->nb_host.variants == 1;
-    if (total) mc_energy_kernel<<<grid_for(total, h->sms), kMcThreads, 0, h->stream>>>(mc_args(h), total < h->n ? h->list : nullptr, total, forward);
+    if (total) {
+        McMasks m;
+        for (int v = 0; v < 6; ++v) m.of[v] = nb_mask(h->nb_host, v);
+        const uint32_t* list = total < h->n ? h->list : nullptr;  // none: every cell in order
+        const int grid = std::min(grid_for(total, h->sms), h->sms * 4);  // more blocks queue at its atomics
+        if (forward) mc_energy_kernel<true><<<grid, kMcThreads, 0, h->stream>>>(mc_args(h), m, list, total);
+        else mc_energy_kernel<false><<<grid, kMcThreads, 0, h->stream>>>(mc_args(h), m, list, total);
+    }
     h->launches += total ? 1 : 0;
     VCA_CUDA(cudaGetLastError());
     VCA_CUDA(cudaStreamSynchronize(h->stream));
