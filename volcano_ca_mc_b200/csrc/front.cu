@@ -806,12 +806,17 @@ __global__ __launch_bounds__(kFrontBatchThreads, 4) void ca_front_batch_kernel(c
 }
 
 // The front list of the current planes: every LAVA cell, 16 cells of a row per thread (a row is a
-// multiple of 64 cells), and with `totals` the LAVA and AIR cells of the grid (countInitialState,
-// LavaCA.hpp:1252-1280).  Reads one byte per cell.
-__global__ __launch_bounds__(256) void ca_front_list_kernel(const __grid_constant__ CaFrontArgs k, uint64_t cells, int totals) {
+// multiple of 64 cells); the scratch of the steps cleared on the way.  With `snap` also the LAVA and AIR
+// cells of the grid and the stop state they give (countInitialState, LavaCA.hpp:1252-1280), which the last
+// block leaves in the control block and in host-mapped memory.  Reads one byte per cell and writes four.
+__global__ __launch_bounds__(256) void ca_front_list_kernel(const __grid_constant__ CaFrontArgs k, uint64_t cells, int t0, CaCtrl* snap) {
     const int lane = threadIdx.x & 31;
-    const uint64_t chunks = cells / 16, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t chunks = cells / 16, stride = (uint64_t)gridDim.x * blockDim.x, me = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     unsigned long long air = 0;
+    for (uint64_t i = me; i < cells / 4; i += stride) reinterpret_cast<uint4*>(k.mark)[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = me; i < (uint64_t)k.g.nx * k.g.ny; i += stride) k.stamp[i] = 0xFFFFFFFFu;  // no step
+    if (snap)  // the steps to come add their totals up in the histories
+        for (int64_t t = t0 + (int64_t)me; t < k.max_steps; t += stride) k.hist_active[t] = k.hist_changed[t] = 0;
     for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < chunks; base += stride) {  // uniform over the block
         const uint64_t ch = base + threadIdx.x;
         uint32_t w[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
@@ -847,9 +852,32 @@ __global__ __launch_bounds__(256) void ca_front_list_kernel(const __grid_constan
             ++at;
         }
     }
-    if (!totals) return;
+    if (!snap) return;
     const unsigned a = __reduce_add_sync(0xFFFFFFFFu, (unsigned)air);
-    if (lane == 0 && a) atomicAdd(&k.ctrl->acc_born, (unsigned long long)a);
+    CaCtrl* ctrl = k.ctrl;
+    if (lane == 0 && a) atomicAdd(&ctrl->acc_born, (unsigned long long)a);
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    unsigned left = 0;
+    if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(left) : "l"(&ctrl->front_exit) : "memory");
+    if (__shfl_sync(0xFFFFFFFFu, left, 0) != gridDim.x - 1u) return;
+    if (lane == 0) {  // the last block: LavaCA::countInitialState (LavaCA.hpp:1272-1279)
+        const uint64_t lava = __ldcg(&ctrl->front_n), none = __ldcg(&ctrl->acc_born);
+        int stop = VCA_STOP_RUNNING;
+        if (!k.classic && lava == 0) stop = VCA_STOP_NO_LAVA;
+        else if (k.classic && none == 0) stop = VCA_STOP_NO_AIR;
+        else if (k.max_steps <= t0) stop = VCA_STOP_MAX_STEPS;
+        ctrl->front_exit = 0;
+        ctrl->acc_born = 0;
+        ctrl->lava = lava;
+        ctrl->air = none;
+        ctrl->stop = stop;
+        __threadfence();
+    }
+    __syncwarp();
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(ctrl);
+    volatile uint32_t* to = reinterpret_cast<volatile uint32_t*>(snap);
+    for (int i = lane; i < (int)(sizeof(CaCtrl) / sizeof(uint32_t)); i += 32) to[i] = __ldcg(from + i);
 }
 
 // ============================================================================================
@@ -908,27 +936,23 @@ CaFrontArgs front_args(const vca_ca* h) {
     return k;
 }
 
-static vca_status front_list_launch(vca_ca* h, int totals) {
-    VCA_CUDA(cudaMemsetAsync(h->flow[h->front_buf ^ 1], 0, 4 * h->plane_cells, h->stream));
-    VCA_CUDA(cudaMemsetAsync(h->heights_dev, 0xFF, sizeof(int32_t) * (size_t)h->geom.nx * h->geom.ny, h->stream));  // no step
-    VCA_CUDA(cudaMemsetAsync(&h->ctrl->front_n, 0, 2 * sizeof(uint32_t), h->stream));  // and front_prev
+static vca_status front_list_launch(vca_ca* h, int t0, CaCtrl* snap) {
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((h->plane_cells / 16 + 255) / 256, (uint64_t)h->sms * 8));
-    ca_front_list_kernel<<<blocks, 256, 0, h->stream>>>(front_args(h), h->plane_cells, totals);
+    ca_front_list_kernel<<<blocks, 256, 0, h->stream>>>(front_args(h), h->plane_cells, t0, snap);
     VCA_CUDA(cudaGetLastError());
     h->launches += 1;
     h->front_listed = true;
     return VCA_OK;
 }
-vca_status front_init(vca_ca* h, int steps_done) {
-    // the steps to come add their totals up in the histories
-    const size_t ahead = (size_t)std::max(0, h->desc.max_steps - steps_done);
-    if (ahead) {
-        VCA_CUDA(cudaMemsetAsync(h->hist_active + steps_done, 0, 8 * ahead, h->stream));
-        VCA_CUDA(cudaMemsetAsync(h->hist_changed + steps_done, 0, 8 * ahead, h->stream));
-    }
-    return front_list_launch(h, 1);
+
+// The list, the totals and the stop state of the current buffer, for a control block that is zero but for
+// its step and its rules; left in the host's mirror.
+vca_status front_init(vca_ca* h, int steps_done) { return front_list_launch(h, steps_done, h->ctrl_host_dev); }
+// The list alone.
+vca_status front_list(vca_ca* h) {
+    VCA_CUDA(cudaMemsetAsync(&h->ctrl->front_n, 0, 2 * sizeof(uint32_t), h->stream));  // and front_prev
+    return front_list_launch(h, 0, nullptr);
 }
-vca_status front_list(vca_ca* h) { return front_list_launch(h, 0); }
 
 int front_batch_grid(int sms) {
     int per_sm = 0;

@@ -258,6 +258,8 @@ struct vca_ca {
     int graph_grid = 0, graph_cand = 0;
     vca::CaCtrl* ctrl_ring = nullptr;       // pinned, host-mapped: two in-flight copies of the control block
     vca::CaCtrl* ctrl_ring_dev = nullptr;   // its device address
+    unsigned long long* hist_mapped = nullptr;      // host-mapped room for the histories of a short run
+    unsigned long long* hist_mapped_dev = nullptr;  // its device address
     cudaEvent_t ring_ev[2] = {nullptr, nullptr};
     vca_ca_batch* batch = nullptr;          // the batch stepping this handle, if any (vca_ca_batch_add)
     int batch_slot = -1;
@@ -276,8 +278,8 @@ struct vca_ca {
 namespace vca {
 // front.cu: the front form of the ACTIVE schedule
 CaFrontArgs front_args(const vca_ca* h);
-vca_status front_init(vca_ca* h, int steps_done);                   // marks cleared, list and totals from the planes
-vca_status front_list(vca_ca* h);                                   // the same, the totals kept
+vca_status front_init(vca_ca* h, int steps_done);                   // scratch cleared, list, totals and stop state from the planes
+vca_status front_list(vca_ca* h);                                   // scratch cleared, list; the totals kept
 vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop);
 int front_batch_grid(int sms);                                      // blocks of a batched launch, 0 on failure
 cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cudaStream_t stream);
