@@ -1122,6 +1122,78 @@ __global__ __launch_bounds__(kThreads, 4) void ca_rules_dyn_kernel(const __grid_
 // finishes the step (finishStep, LavaCA.hpp:1206-1229).
 // ------------------------------------------------------------------------------------------
 constexpr int kCandThreads = 128;
+
+// One candidate by a warp: lane i has the variant's neighbour i, lane 26 the cell two below, lanes 27-30 the
+// cells beside the one below (tryPonding, LavaCA.hpp:443-461); everything is loaded in one round.  The same
+// decision as air_gains_lava.
+__device__ __forceinline__ bool air_gains_lava_warp(const CaKernelArgs& k, const uint8_t* T, const int32_t* F, const float* Te,
+                                                    int x, int y, int z, uint64_t prefix, uint64_t gidx, int lane, int32_t& flow,
+                                                    float& temp) {
+    const CaGeom& g = k.g;
+    const NbTable& nb = k.tables.nb;
+    const uint64_t h = hash_index(prefix, gidx);
+    const int var = nb.variants == 1 ? 0 : (int)fast_mod(hash_salt(h, kSaltNeighborhood), k.var_mod);
+    int dx = 0, dy = 0, dz = 0;
+    bool in = lane < nb.count[var];
+    if (in) {
+        dx = nb.off[var][lane][0], dy = nb.off[var][lane][1], dz = nb.off[var][lane][2];
+    } else if (lane == 26) {
+        in = z >= 2;
+        dz = -2;
+    } else if (lane >= 27 && lane < (g.ny > 1 ? 31 : 29)) {
+        in = z >= 1;
+        dx = lane == 27 ? -1 : lane == 28 ? 1 : 0;
+        dy = lane == 29 ? -1 : lane == 30 ? 1 : 0;
+        dz = -1;
+    }
+    int sx = x + dx, sy = y + dy, sz = z + dz;
+    in = in & resolve1_sel(g, sx, sy, sz);
+    const int64_t self = pidx(g, x, y, z), sp = in ? pidx(g, sx, sy, sz) : self;
+    const int type = __ldg(T + sp);  // (outside the grid: the cell itself, which is AIR)
+    const int32_t fl = __ldg(F + sp);
+    const float te = __ldg(Te + sp);
+    const int d = k.classic ? 0 : (int)__ldg(k.desc + sp);
+    const int c_drop = k.classic ? 0 : (int)k.drop[self];
+    const bool pond = !k.classic && k.ponding && k.spill != nullptr && z >= 1;
+    const int spill = pond ? __ldg(k.spill + x + (int64_t)g.nx * y) : 0;
+    // the cell below is supported: the grid floor, solid ground, or LAVA below the spill level; and closed
+    const int under = __shfl_sync(0xFFFFFFFFu, type, 26);
+    const bool sup = z < 2 || solid_ground(under) || (under == kLava && z - 2 < spill);
+    const unsigned sides = g.ny > 1 ? 0x78000000u : 0x18000000u;
+    const bool closed = (__ballot_sync(0xFFFFFFFFu, in && type != kAir && type != kVoid) & sides) == sides;
+    bool use = in && lane < nb.count[var] && type == kLava;
+    float cooling = 0.0f;
+    if (!k.classic) {
+        if (dz < 0) {
+            use = use && dx == 0 && dy == 0 && pond && z <= spill && sup && closed;
+            cooling = k.cool_lateral;
+        } else if (dz > 0) {
+            use = use && ((dx == 0 && dy == 0) || (d == 1 && c_drop == 0));
+            cooling = k.cool_fall;
+        } else {
+            use = use && d >= 0 && c_drop == d && !(d == 1 && k.diag_falls);
+            cooling = k.cool_lateral;
+        }
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, use);
+    if (m == 0) return false;
+    // the vote (CandidateVote, CaRules.hpp:127-183)
+    const unsigned alike = __match_any_sync(0xFFFFFFFFu, fl) & m;
+    const bool lead = use && lane == __ffs(alike) - 1;
+    const int votes = lead ? __popc(alike) : 0, best = __reduce_max_sync(0xFFFFFFFFu, votes);
+    const unsigned tied = __ballot_sync(0xFFFFFFFFu, lead && votes == best), ties = __popc(tied);
+    const unsigned want = ties > 1 ? (unsigned)(hash_salt(h, kSaltTieBreak) % ties) : 0u;
+    unsigned rank = 0;  // ties: the smallest tied id has rank 0
+    for (unsigned r = tied; r; r &= r - 1) rank += __shfl_sync(0xFFFFFFFFu, fl, __ffs(r) - 1) < fl;
+    const int src = __ffs(__ballot_sync(0xFFFFFFFFu, lead && votes == best && rank == want)) - 1;
+    const float own = k.classic ? 0.0f : __fsub_rn(te, cooling);
+    flow = __shfl_sync(0xFFFFFFFFu, fl, src);
+    temp = __shfl_sync(0xFFFFFFFFu, own, src);
+    for (unsigned r = __shfl_sync(0xFFFFFFFFu, alike, src); r; r &= r - 1) temp = fmaxf(temp, __shfl_sync(0xFFFFFFFFu, own, __ffs(r) - 1));
+    return k.classic || temp >= k.solidus;
+}
+
+template <bool kWarp>
 __device__ __forceinline__ void cand_body(const CaKernelArgs& k, uint32_t bid, uint32_t nblk) {
     __shared__ unsigned long long s_red[kCandThreads / 32];
     __shared__ bool s_last;
@@ -1138,14 +1210,15 @@ __device__ __forceinline__ void cand_body(const CaKernelArgs& k, uint32_t bid, u
     const unsigned n = ctrl->cand_count;
     // the blocks that hold listed cells take part (at least one, which finishes the step); the others
     // leave at once, so a short list costs a few blocks instead of the whole grid
-    const unsigned parts = max(1u, min(nblk, (n + kCandThreads - 1) / kCandThreads));
+    constexpr unsigned kPer = kWarp ? kCandThreads / 32 : kCandThreads;  // candidates of a block in one round
+    const unsigned parts = max(1u, min(nblk, (n + kPer - 1) / kPer));
     if (bid >= parts) return;
     const int lane = threadIdx.x & 31;
     unsigned born = 0;
-    const uint64_t stride = (uint64_t)nblk * kCandThreads;
+    const uint64_t stride = (uint64_t)nblk * kPer;
     // warp-uniform loop (the appends below use full-warp collectives)
-    for (uint64_t base = bid * (uint64_t)kCandThreads; base < n; base += stride) {
-        const uint64_t j = base + threadIdx.x;
+    for (uint64_t base = bid * (uint64_t)kPer + (kWarp ? threadIdx.x >> 5 : 0); base < n; base += stride) {
+        const uint64_t j = kWarp ? base : base + threadIdx.x;
         bool gained = false;
         uint32_t gi = 0, tile = 0;
         unsigned faces = 0;  // of the gained cell in its tile
@@ -1157,7 +1230,10 @@ __device__ __forceinline__ void cand_body(const CaKernelArgs& k, uint32_t bid, u
             const int z = (int)(r / (uint32_t)g.ny);
             int32_t nf;
             float nt;
-            if (air_gains_lava(k, T, F, Te, x, y, z, prefix, gi + k.gidx_base, &nf, &nt)) {
+            bool gains;
+            if constexpr (kWarp) gains = air_gains_lava_warp(k, T, F, Te, x, y, z, prefix, gi + k.gidx_base, lane, nf, nt) && lane == 0;
+            else gains = air_gains_lava(k, T, F, Te, x, y, z, prefix, gi + k.gidx_base, &nf, &nt);
+            if (gains) {
                 const int64_t p = pidx(g, x, y, z);
                 k.type[nxt][p] = kLava;
                 k.flow[nxt][p] = nf;
@@ -1229,8 +1305,19 @@ __device__ __forceinline__ void cand_body(const CaKernelArgs& k, uint32_t bid, u
         ctrl->steps = steps;  // read by the next kernels, after this launch has completed
     }
 }
+// A warp per candidate while the list is short: a thread then goes through some 2000 instructions one after
+// another for a cell with a handful of warps on its SM, a warp through a tenth of that with one round of
+// loads.  With events around it the pass over some 10^4 candidates takes 27 us by threads and 13.4 by warps
+// (256 x 256 x 128), over some 10^5 (classic 200^3) 97 by threads and 200 by warps.  Classic 128^3, whose list
+// grows from one to the other, takes 26.0 us a pass by threads and 25.0 / 25.1 / 26.0 / 30.2 with the line at
+// 2 / 4 / 8 / 16 candidates per warp; 512 x 512 x 128 with 200 vents 29.9 and 24.6 / 22.5 / 22.2 / 22.1.
+constexpr unsigned kCandWarpMost = 4 * (kCandThreads / 32);
+__device__ __forceinline__ void cand_pass(const CaKernelArgs& k, uint32_t bid, uint32_t nblk) {
+    if (k.ctrl->cand_count <= kCandWarpMost * nblk) cand_body<true>(k, bid, nblk);
+    else cand_body<false>(k, bid, nblk);
+}
 __global__ __launch_bounds__(kCandThreads, 4) void ca_cand_kernel(const __grid_constant__ CaKernelArgs k) {
-    cand_body(k, blockIdx.x, gridDim.x);
+    cand_pass(k, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1422,7 +1509,7 @@ __global__ __launch_bounds__(kCandThreads, 4) void ca_cand_batch_kernel(const __
     if (m.x < 0) return;
     __shared__ __align__(16) CaKernelArgs s_k;
     load_args(s_k, b.args[m.x]);
-    cand_body(s_k, (uint32_t)m.y, (uint32_t)b.cand_n[m.x]);
+    cand_pass(s_k, (uint32_t)m.y, (uint32_t)b.cand_n[m.x]);
 }
 
 // Stop state of every member after a round of steps and the size of its next one (tiles, or cells of
@@ -1676,9 +1763,10 @@ vca_status init_state(vca_ca* h, int steps_done) {
 }
 
 // The rules pass of the handle's tile-shape family.
-// Tiles handed out at run time pay where a block has many tiles of uneven cost: DENSE with at
-// least 64 tiles per block (measured: c3 DENSE -20 %; with 14 tiles per block, c2, +12 %).
-constexpr uint64_t kDynTilesPerBlock = 64;
+// Tiles handed out at run time pay where a block has enough tiles to even out.  DENSE, 60 steps, by the grid /
+// at run time: 14 tiles per block (256 x 256 x 128) 4.38 / 4.34 ms, 22 5.79 / 5.37, 55 (512 x 512 x 128)
+// 11.26 / 10.17, 111 20.4 / 18.0; with one tile per block (64^3) the pass takes 14.0 / 15.4 us.
+constexpr uint64_t kDynTilesPerBlock = 16;
 
 template <class S>
 void launch_rules_shape(const vca_ca* h, const CaKernelArgs& k) {
