@@ -29,8 +29,8 @@
 // some 7 us with all SMs and 5 us in one block, whose barriers are __syncthreads; above that the list
 // stream (9 bytes per LAVA cell from L2).  Against the tile schedule on one B200: 1024 x 1024 x 256,
 // 800 steps, up to 1.0 M LAVA cells 208 -> 13.8 ms; 256 x 256 x 128, 400 steps 14.9 -> 2.8 ms;
-// 512 x 1 x 256, 300 steps 8.1 -> 1.54 ms; classic 100^3, 70 steps 2.4 -> 1.2 ms; ten mixed jobs in a
-// batch 19.8 -> 6.1 ms.  Three forms brought the last part of it (mid: 256 x 256 x 128, 3.3 -> 2.8 ms):
+// 512 x 1 x 256, 300 steps 8.1 -> 1.45 ms; classic 100^3, 70 steps 2.4 -> 1.2 ms; ten mixed jobs in a
+// batch 19.8 -> 4.1 ms.  Three forms brought the last part of it (mid: 256 x 256 x 128, 3.3 -> 2.8 ms):
 // slots held in registers while each thread has at most one; a block's births counted in shared memory, so
 // that each block takes its slots of the list with one atomic; and votes among five and more sources of
 // several flows by a warp, one lane per source (one thread counting them in local arrays held up the second
@@ -965,12 +965,13 @@ cudaError_t front_batch_launch(const CaFrontBatch& view, int grid, int steps, cu
     return cudaLaunchCooperativeKernel((const void*)ca_front_batch_kernel, grid, kFrontBatchThreads, args, 0, stream);
 }
 
-constexpr int kFrontChunk = 64;        // steps per launch of a run
+constexpr int kFrontChunk = 256;       // most steps per launch of a run (64: 1 % slower)
 
-// The launch for a list of n slots.  Up to kFrontSolo one small block: its step has no grid barrier and each
-// of its barriers waits for 8 warps only (512 x 1 x 256, 300 steps: 1.54 ms; left to all SMs above 256 slots
-// 1.84 ms; one block of 1024 threads 1.9 ms).  Up to kFrontSmall blocks of 256 threads on all SMs, which hold
-// a slot per thread in registers up to 37 888 slots; beyond, the list is streamed and 1024 threads stream it
+// The launch for a list of n slots.  Up to kFrontSolo one block with a thread per slot, which keeps it in
+// registers: its step has no grid barrier, and its barriers wait for no more warps than needed (512 x 1 x 256,
+// 300 steps, up to 513 slots: 1.45 ms; 256 threads that stream the list beyond 256 slots 1.60 ms; all SMs
+// beyond 256 slots 1.84 ms; one block of 1024 threads 1.9 ms).  Up to kFrontSmall blocks of 256 threads on all
+// SMs, which hold a slot per thread up to 37 888 slots; beyond, the list is streamed and 1024 threads stream it
 // faster (256 x 256 x 128, 400 steps: 2.80 ms with the line at 40 000, 2.98 ms without the small blocks;
 // classic 100^3: 1.21 ms, with the line at 160 000 1.34 ms).  A launch ends early when its list has
 // outgrown `most`.
@@ -980,7 +981,8 @@ struct FrontShape {
     uint32_t most;
 };
 static FrontShape front_shape(const vca_ca* h, uint64_t n) {
-    if (n <= kFrontSolo) return {256, 1, kFrontSolo};
+    if (n <= kFrontSolo / 2) return {256, 1, kFrontSolo / 2};
+    if (n <= kFrontSolo) return {512, 1, kFrontSolo};
     if (n <= kFrontSmall) return {256, h->sms, 2 * kFrontSmall};
     return {kFrontThreads, h->sms, 0xFFFFFFFFu};
 }
@@ -995,9 +997,9 @@ vca_status front_run(vca_ca* h, int max_new_steps, bool until_stop) {
         const FrontShape f = front_shape(h, n);
         uint32_t most = until_stop ? f.most : 0xFFFFFFFFu;
         CaCtrl* snap = h->ctrl_ring_dev + slot;
-        const bool small = f.threads == 256;
-        const auto kernel = small ? (k.classic ? ca_front_kernel<256, true> : ca_front_kernel<256, false>)
-                                  : (k.classic ? ca_front_kernel<kFrontThreads, true> : ca_front_kernel<kFrontThreads, false>);
+        const auto kernel = f.threads == 256   ? (k.classic ? ca_front_kernel<256, true> : ca_front_kernel<256, false>)
+                            : f.threads == 512 ? (k.classic ? ca_front_kernel<512, true> : ca_front_kernel<512, false>)
+                                               : (k.classic ? ca_front_kernel<kFrontThreads, true> : ca_front_kernel<kFrontThreads, false>);
         if (f.blocks == 1) {
             kernel<<<1, f.threads, 0, h->stream>>>(k, steps, most, snap);
             VCA_CUDA(cudaGetLastError());
