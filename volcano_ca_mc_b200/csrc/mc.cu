@@ -1390,17 +1390,22 @@ __device__ __forceinline__ void gr_union(uint32_t* parent, uint32_t a, uint32_t 
     atomicOr(err, 1u);
 }
 
+// Threads of a block of the grain pass: its grid barriers cost an arrival per block, so fewer and larger blocks
+// are faster until they leave SMs without one.  50^3 after 90 MCS, by 256 / 512 / 1024 threads: 64 / 52 / 52 us
+// a call; 128^3 456 / 390 / 356; 30^3 40 / 42 / 43; 81 K listed cells 45 / 46 / 55.
+constexpr int kGrainThreads = 512;
+
 // All passes in one cooperative launch (a grid barrier after each): every cell under its run in x; unions
 // over the forward offsets of the connectivity (dz, dy, dx order) on the axes of size > 1; sizes and high
 // cells per root; the statistics, summed per block before they reach the counters.  The last block hands
 // them to the host (out: host-mapped).  With a few 10^5 cells the four passes are latencies; separate
 // launches with an atomic per thread and counter took 2.05 ms a call for 401 K cells and 0.18 ms for 50^3,
-// this one 0.094 and 0.064 ms (0.039 before the first sweep: what is left grows with the unions).
-__global__ __launch_bounds__(kMcThreads) void mc_grains_kernel(const __grid_constant__ McArgs a, const uint32_t* list,
+// this one 0.088 and 0.052 ms (0.035 before the first sweep: what is left grows with the unions).
+__global__ __launch_bounds__(kGrainThreads) void mc_grains_kernel(const __grid_constant__ McArgs a, const uint32_t* list,
                                                                uint64_t count, int moore, const float* mob, double threshold,
                                                                uint32_t* parent, uint32_t* gsize, uint32_t* ghigh, GrainAcc* acc,
                                                                GrainAcc* out) {
-    const uint64_t i0 = blockIdx.x * (uint64_t)kMcThreads + threadIdx.x, T = (uint64_t)gridDim.x * kMcThreads;
+    const uint64_t i0 = blockIdx.x * (uint64_t)kGrainThreads + threadIdx.x, T = (uint64_t)gridDim.x * kGrainThreads;
     const int lane = threadIdx.x & 31;
     // a cell starts under the first cell of its run of one orientation in x, as far as the warp (in cell
     // order) or four cells (a list) show it; rows that wrap are united below
@@ -2564,8 +2569,8 @@ vca_status vca_mc_grains(vca_mc* h, int moore, double mobility_threshold, vca_mc
         VCA_CUDA(cudaMalloc(&h->ghigh, 4 * h->cap_n));
         VCA_CUDA(cudaMalloc(&h->gacc, sizeof(GrainAcc)));
         VCA_CUDA(cudaMemsetAsync(h->gacc, 0, sizeof(GrainAcc), h->stream));
-        VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h->grain_per_sm, mc_grains_kernel, kMcThreads, 0));
-        h->grain_per_sm = std::max(1, std::min(h->grain_per_sm, 4));  // more blocks lengthen its barriers
+        VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h->grain_per_sm, mc_grains_kernel, kGrainThreads, 0));
+        h->grain_per_sm = std::max(1, std::min(h->grain_per_sm, 4 * 256 / kGrainThreads));  // more blocks lengthen its barriers
     }
     GrainAcc* acc = static_cast<GrainAcc*>(h->gacc);
     uint64_t total = h->color_off.back();
@@ -2573,11 +2578,11 @@ vca_status vca_mc_grains(vca_mc* h, int moore, double mobility_threshold, vca_mc
     const float* mob = h->mobility_set ? h->mobility : nullptr;
     *h->gacc_host = GrainAcc{};
     if (total) {
-        const int grid = (int)std::min<uint64_t>((total + kMcThreads - 1) / kMcThreads, (uint64_t)h->sms * h->grain_per_sm);
+        const int grid = (int)std::min<uint64_t>((total + kGrainThreads - 1) / kGrainThreads, (uint64_t)h->sms * h->grain_per_sm);
         const uint32_t* list = total < h->n ? h->list : nullptr;  // none: every cell in order (also where there is a list)
         GrainAcc* out = h->gacc_host_dev;
         void* args[] = {&a, &list, &total, &moore, &mob, &mobility_threshold, &h->gparent, &h->gsize, &h->ghigh, &acc, &out};
-        VCA_CUDA(cudaLaunchCooperativeKernel((const void*)mc_grains_kernel, grid, kMcThreads, args, 0, h->stream));
+        VCA_CUDA(cudaLaunchCooperativeKernel((const void*)mc_grains_kernel, grid, kGrainThreads, args, 0, h->stream));
         h->launches += 1;
     }
     VCA_CUDA(cudaStreamSynchronize(h->stream));
