@@ -97,3 +97,23 @@ def test_small_spaces_match_oracle(case):
     info = mc.info()
     assert (info.attempts, info.accepted, info.uphill, info.sweeps) == (*(int(v) for v in tot), done)
     mc.close()
+
+
+@pytest.mark.parametrize("dims", [(128, 95, 98), (128, 96, 99), (300, 160, 51)], ids=lambda d: "x".join(map(str, d)))
+def test_space_block_sizes_match_oracle(dims):
+    """Spaces below, at and above a group of eight cells per thread of the large blocks (148 x 512 groups a colour)."""
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    domain = np.ones(n, np.uint8)
+    for nb, Q in (("moore", 200), ("von_neumann", 20)):
+        mp = O.mc_params(nx, ny, nz, nb, "absorbing", True, 5, Q, 1.0, 0.6)
+        spin = O.mc_init(mp, domain)
+        mc = capi.PottsMC(capi.McParams(nx, ny, nz, neighborhood=nb, boundary="absorbing", domain_full=True, seed=5, Q=Q, kT=0.6))
+        mc.set_domain(None)
+        mc.initialize()
+        tot = np.zeros(3, np.uint64)
+        for done in range(2):
+            tot += O.mc_sweep(mp, done, domain, None, spin)
+        assert mc.sweep(2) == int(tot[1])
+        assert np.array_equal(mc.crystals(), spin)
+        mc.close()

@@ -668,11 +668,15 @@ __global__ __launch_bounds__(kMcThreads, 2) void mc_sweeps_kernel(const __grid_c
 // neighbour of x = 0 on a wrapped axis), nx cells, the orientation at x = 0, and room for the last load.
 // What bounds it: the integer ALU (79 % busy), three 64-bit hashes of a trial (two at kT = 0) above all.
 // Per MCS on one B200 against a thread per cell with 26 byte loads and compares (709 instructions per
-// trial): 512 x 512 x 256 Moore, Q = 64, kT = 0.5 1.80 -> 0.79 ms, the same von Neumann 1.88 -> 0.54 ms,
+// trial): 512 x 512 x 256 Moore, Q = 64, kT = 0.5 1.80 -> 0.73 ms, the same von Neumann 1.88 -> 0.54 ms,
 // 256 x 256 x 128 pentagonal 0.30 -> 0.16 ms, 100^3 Moore 38 -> 31 us.  Three resident blocks per SM
 // instead of two (80 registers, spills) 0.85 ms; moving adds and shifts to the FMA pipe 0.89 ms.
 // ------------------------------------------------------------------------------------------
-constexpr int kSpaceBlocks = 2;  // resident blocks per SM the registers are limited to
+// Threads of a block (kThreads): one block of 512 per SM where a colour has a group for each of their threads
+// (half the arrivals at the barriers: 512 x 512 x 256, 10 MCS 7.95 -> 7.39 ms, 200^3 pentagonal, 40 MCS 6.24 ->
+// 6.01), else blocks of 128, which reach more SMs (80^3 1.21 -> 1.02 ms, 120^3 1.66 -> 1.43; by 512 1.67, 1.66).
+constexpr int kSpaceThreads = 512, kSpaceSmall = 128;
+constexpr int kSpaceResident = 512;  // threads of an SM the registers are limited to
 struct McSpace {
     uint8_t* sp;             // P8-byte rows: orientation - 1
     const float* mob;        // mobility of every cell (kMobility)
@@ -786,12 +790,12 @@ __device__ __forceinline__ uint32_t add_planes(const Planes& a, const Planes& b,
 
 // kNb: 0 the whole 3 x 3 x 3 block (Moore), 1 the six faces (von Neumann), 2 by the variants' masks.
 // kWide: Q > 128, so an orientation - 1 takes all eight bits of its byte.
-template <bool kMobility, int kNb, bool kParity, bool kWide>
-__global__ __launch_bounds__(kMcThreads, kSpaceBlocks) void mc_space_sweeps_kernel(const __grid_constant__ McArgs a,
+template <bool kMobility, int kNb, bool kParity, bool kWide, int kThreads>
+__global__ __launch_bounds__(kThreads, kSpaceResident / kThreads) void mc_space_sweeps_kernel(const __grid_constant__ McArgs a,
                                                                         const __grid_constant__ McSpace d, int sweeps) {
     __shared__ unsigned long long s_table[kTableSide * kTableSide];
-    __shared__ unsigned long long s_red[3][kMcThreads / 32];
-    for (int i = threadIdx.x; i < kTableSide * kTableSide; i += kMcThreads) {
+    __shared__ unsigned long long s_red[3][kThreads / 32];
+    for (int i = threadIdx.x; i < kTableSide * kTableSide; i += kThreads) {
         // (r >> 11) < th is r < th << 11 as long as that fits
         const unsigned long long th = a.table[i];
         s_table[i] = th >> 63 ? 1ull : (th >> 53 ? 2ull : th << 11);
@@ -799,7 +803,7 @@ __global__ __launch_bounds__(kMcThreads, kSpaceBlocks) void mc_space_sweeps_kern
     __syncthreads();
     McCtrl* ctrl = a.ctrl;
     const uint32_t t0 = ctrl->sweeps;
-    const uint32_t T = gridDim.x * kMcThreads, me = blockIdx.x * kMcThreads + threadIdx.x;
+    const uint32_t T = gridDim.x * kThreads, me = blockIdx.x * kThreads + threadIdx.x;
     const int colors = kParity ? 2 : a.classes[0] * a.classes[1] * a.classes[2];
     unsigned long long sum_att = 0, sum_acc = 0, sum_up = 0;
     uint32_t my_att = 0, my_acc = 0, my_up = 0;  // of one sweep
@@ -1047,7 +1051,7 @@ __global__ __launch_bounds__(kMcThreads, kSpaceBlocks) void mc_space_sweeps_kern
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long sa = 0, sc = 0, su = 0;
-        for (int w = 0; w < kMcThreads / 32; ++w) {
+        for (int w = 0; w < kThreads / 32; ++w) {
             sa += s_red[0][w];
             sc += s_red[1][w];
             su += s_red[2][w];
@@ -1894,18 +1898,19 @@ vca_status sweeps_launch_shape(vca_mc* h, SweepsKernel kernel, McColors* col, in
 
 using SpaceKernel = void (*)(McArgs, McSpace, int);
 
-template <bool kMobility, bool kWide>
+template <bool kMobility, bool kWide, int kThreads>
 SpaceKernel space_kernel_of(const vca_mc* h) {
-    if (h->parity_colors) return mc_space_sweeps_kernel<kMobility, 1, true, kWide>;
+    if (h->parity_colors) return mc_space_sweeps_kernel<kMobility, 1, true, kWide, kThreads>;
     switch (h->desc.neighborhood) {
-        case VCA_NB_MOORE: return mc_space_sweeps_kernel<kMobility, 0, false, kWide>;
-        case VCA_NB_VON_NEUMANN: return mc_space_sweeps_kernel<kMobility, 1, false, kWide>;
-        default: return mc_space_sweeps_kernel<kMobility, 2, false, kWide>;
+        case VCA_NB_MOORE: return mc_space_sweeps_kernel<kMobility, 0, false, kWide, kThreads>;
+        case VCA_NB_VON_NEUMANN: return mc_space_sweeps_kernel<kMobility, 1, false, kWide, kThreads>;
+        default: return mc_space_sweeps_kernel<kMobility, 2, false, kWide, kThreads>;
     }
 }
+template <int kThreads>
 SpaceKernel space_kernel_of(const vca_mc* h) {
-    if (h->desc.Q > 128) return h->mobility_on ? space_kernel_of<true, true>(h) : space_kernel_of<false, true>(h);
-    return h->mobility_on ? space_kernel_of<true, false>(h) : space_kernel_of<false, false>(h);
+    if (h->desc.Q > 128) return h->mobility_on ? space_kernel_of<true, true, kThreads>(h) : space_kernel_of<false, true, kThreads>(h);
+    return h->mobility_on ? space_kernel_of<true, false, kThreads>(h) : space_kernel_of<false, false, kThreads>(h);
 }
 
 // Bytes of a row of the byte copy: 8 in front, the cells, 8 behind.
@@ -2058,12 +2063,13 @@ vca_status sp8_reserve(vca_mc* h, uint64_t bytes) {
 // Whether the byte form of the list sweeps applies, and its launch: Q <= 256, orientations as
 // vca_mc_initialize and the sweeps left them (only the domain's cells are copied, so a value set outside
 // of it would be missed), 32-bit offsets, rows not too short for their frame columns, and every block's
-// entries in shared memory.  At least 128 threads per block, then one block per SM.
+// entries in shared memory.  At least 96 threads per block, then one block per SM
+// (81 K cells, 400 passes: 1.92 ms; by 128 threads 1.96, 192 2.14, 256 2.24).
 bool list_bytes_shape(const vca_mc* h, McColors* col, int* grid, int* threads, size_t* smem) {
     if (h->desc.Q > 256 || h->slab_zoff >= 0 || h->user_spins || h->desc.nx < 6 || list_bytes(h) > 0xFFFFFFF0ull) return false;
     uint64_t widest = 1;
     for (int c = 0; c < h->colors; ++c) widest = std::max<uint64_t>(widest, h->color_off[c + 1] - h->color_off[c]);
-    const uint64_t g = std::min<uint64_t>((widest + 127) / 128, (uint64_t)h->sms);
+    const uint64_t g = std::min<uint64_t>((widest + 95) / 96, (uint64_t)h->sms);
     const uint64_t t = std::min<uint64_t>(((widest + g - 1) / g + 31) / 32 * 32, (uint64_t)kListThreads - 32);
     int total = 0;
     for (int c = 0; c < h->colors; ++c) {
@@ -2405,19 +2411,19 @@ vca_status vca_mc_sweep(vca_mc* h, int count, uint64_t* accepted) {
             const uint64_t rows = (uint64_t)va.ny * va.nz, bytes = (uint64_t)d.P8 * rows;
             if (vca_status s = sp8_reserve(h, bytes)) return s;
             d.sp = h->sp8;
-            SpaceKernel sk = space_kernel_of(h);
-            int per_sm = 0;
-            VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sk, kMcThreads, 0));
-            // no more blocks than the largest colour has groups for
+            // groups of the largest colour: no more blocks than they fill
             const uint64_t most = (uint64_t)d.gx[0] * (uint64_t)d.cnt[1][0] * (uint64_t)d.cnt[2][0];
-            const int sgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((most + kMcThreads - 1) / kMcThreads,
-                                                                           (uint64_t)h->sms * std::max(1, per_sm)));
+            const int threads = most >= (uint64_t)h->sms * kSpaceThreads ? kSpaceThreads : kSpaceSmall;
+            SpaceKernel sk = threads == kSpaceThreads ? space_kernel_of<kSpaceThreads>(h) : space_kernel_of<kSpaceSmall>(h);
+            int per_sm = 0;
+            VCA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sk, threads, 0));
+            const int sgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((most + threads - 1) / threads, (uint64_t)h->sms * std::max(1, per_sm)));
             const int blocks = grid_for(bytes / 8, h->sms);
             mc_pack8_kernel<<<blocks, 256, 0, h->stream>>>(h->spin, h->sp8, va.nx, d.P8, rows);
             VCA_CUDA(cudaGetLastError());
             int n = count;
             void* args[] = {&va, &d, &n};
-            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)sk, sgrid, kMcThreads, args, 0, h->stream));
+            VCA_CUDA(cudaLaunchCooperativeKernel((const void*)sk, sgrid, threads, args, 0, h->stream));
             mc_unpack8_kernel<<<blocks, 256, 0, h->stream>>>(h->sp8, h->spin, va.nx, d.P8, rows);
             VCA_CUDA(cudaGetLastError());
             h->launches += 3;
