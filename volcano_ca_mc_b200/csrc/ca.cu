@@ -2831,6 +2831,7 @@ struct vca_ca_batch {
     bool resplit = false;         // only the split of the blocks is
     int front_chunk = 1;          // steps of the next front launch
     bool round_end[2] = {};       // whether the status in the ring slot ends a round
+    std::vector<std::pair<vca_ca*, int4>> leaving;  // members found stopped at a round's end, with their status
     int pending = -1;             // ring slot whose status is not read yet
     int ring = 0;
     uint64_t graphs = 0, launches = 0;
@@ -2972,23 +2973,21 @@ vca_status batch_detach(vca_ca_batch* b, vca_ca* h, const int4* st) {
     return VCA_OK;
 }
 
-// Reads the status of the graph in ring slot r (waits for it) and takes the members that stopped
-// out of the batch.
+// Reads the status in ring slot r (waits for it): the weights for the split of the blocks and, at the end of a
+// round, the members that stopped (batch_release).
 vca_status batch_collect(vca_ca_batch* b, int r) {
     VCA_CUDA(cudaEventSynchronize(b->status_ev[r]));
-    bool grew = false;
     const int4* st = b->h_status + (size_t)r * b->cap;
+    bool grew = false;
     for (int i = 0; i < b->cap; ++i) {
         vca_ca* h = b->snap[r][(size_t)i];
         if (!h || b->slots[(size_t)i] != h || st[i].x < 0) continue;
         if (st[i].x != VCA_STOP_RUNNING || st[i].y != 0) {
-            if (!b->round_end[r]) continue;  // members leave between rounds
-            if (vca_status s = batch_detach(b, h, &st[i])) return s;
-            b->done.push_back(h);
+            if (b->round_end[r]) b->leaving.push_back({h, st[i]});
             continue;
         }
         // the blocks follow the work: re-split when a member's visited tiles moved by more than 1/8, or
-        // the blocks its front list can use by more than a quarter
+        // when its front list comes near to outgrowing its blocks
         const uint64_t now = std::max<uint64_t>(1, (uint64_t)(uint32_t)st[i].w);
         uint64_t& was = b->weight[(size_t)i];
         const bool moved = h->front ? front_share(now + now / 4) > front_want(was) || 2 * now < was
@@ -3000,6 +2999,16 @@ vca_status batch_collect(vca_ca_batch* b, int r) {
         }
     }
     b->front_chunk = grew ? kFrontBatchFirst : std::min(2 * b->front_chunk, kGraphSteps);
+    return VCA_OK;
+}
+// The members that the last collected rounds found stopped leave, once the round after is launched.
+vca_status batch_release(vca_ca_batch* b) {
+    for (const auto& l : b->leaving) {
+        if (l.first->batch != b) continue;
+        if (vca_status s = batch_detach(b, l.first, &l.second)) return s;
+        b->done.push_back(l.first);
+    }
+    b->leaving.clear();
     return VCA_OK;
 }
 
@@ -3217,11 +3226,13 @@ vca_status vca_ca_batch_advance(vca_ca_batch* b, int max_graphs, vca_ca** finish
             }
             b->pending = r;
         }
+        if (vca_status s = batch_release(b)) return s;
         b->graphs += 1;
     }
     // with nothing left to launch, the last graph's status is read now
     if (b->done.empty() && b->pending >= 0) {
         if (vca_status s = batch_collect(b, b->pending)) return s;
+        if (vca_status s = batch_release(b)) return s;
         b->pending = -1;
     }
     int n = 0;
