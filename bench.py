@@ -683,7 +683,7 @@ def ours(args):
         "e2e": {"value": world * w.cells * e2e_steps / (e2e_ms * 1e-3), "unit": "cell-updates/s",
                 "h2d_bytes_per_step": e2e_h2d, "d2h_bytes_per_step": e2e_d2h, "ms_per_step": e2e_ms / e2e_jobs,
                 "jobs": e2e_jobs, "jobs_in_flight": E2E_INFLIGHT, "phases_median": e2e_phases,
-                "path": "per job: vca_ca_reset + apply_terrain (host priority flood + upload) + place_seeds + run + "
+                "path": "per job: vca_ca_reset + apply_terrain (upload + flood) + place_seeds + run + "
                         "download of the five planes into pinned memory; resident handles each driven by a host "
                         "thread, one run at a time (a job's download and the next job's upload overlap the running "
                         "job); host wall clock over all jobs, first job's upload and last job's download included",

@@ -666,7 +666,7 @@ __global__ __launch_bounds__(kMcThreads, 2) void mc_sweeps_kernel(const __grid_c
 //
 // The copy has rows of P8 bytes: 8 in front (the last one holds the orientation at x = nx - 1, the left
 // neighbour of x = 0 on a wrapped axis), nx cells, the orientation at x = 0, and room for the last load.
-// What bounds it: the integer ALU (79 % busy), three 64-bit hashes of a trial (two at kT = 0) above all.
+// What bounds it: the integer ALU (84 % busy), three 64-bit hashes of a trial (two at kT = 0) above all.
 // Per MCS on one B200 against a thread per cell with 26 byte loads and compares (709 instructions per
 // trial): 512 x 512 x 256 Moore, Q = 64, kT = 0.5 1.80 -> 0.73 ms, the same von Neumann 1.88 -> 0.54 ms,
 // 256 x 256 x 128 pentagonal 0.30 -> 0.16 ms, 100^3 Moore 38 -> 31 us.  Three resident blocks per SM
