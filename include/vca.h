@@ -204,7 +204,7 @@ void vca_ca_destroy(vca_ca* ca);
  * (engine/src/app/Batch.cpp:186-246) starts one engine process per config, one after another, and
  * each LavaCA::run (LavaCA.hpp:253-256) steps one grid.  A batch steps every member grid -- of any
  * size, 2D or 3D, neighbourhood, boundary, seed or schedule -- with shared launches (each block of a
- * launch works on one member): one launch of 16 steps for the ACTIVE members, three launches per
+ * launch works on one member): launches of 2 to 16 steps, 16 in a round, for the ACTIVE members, three per
  * step, captured as a CUDA graph of 16 steps, for the others.  Each member ends exactly as it would alone (same planes, histories and stop step).
  * ---------------------------------------------------------------------------------------- */
 

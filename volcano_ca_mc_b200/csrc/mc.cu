@@ -1077,7 +1077,7 @@ __global__ __launch_bounds__(kThreads, kSpaceResident / kThreads) void mc_space_
 // funnel shift; the unlike bits of the nine rows are added with bitwise adders and counted.
 // Measured on one B200 against 27 loads of 32-bit orientations per trial: 401 K cells, 200 MCS of 8
 // colours 7.04 -> 5.03 ms (3.1 us a pass, of which the release about 0.6 and the loads 1.0), 81 K cells,
-// 100 MCS in four calls 2.73 -> 1.97 ms.
+// 100 MCS in four calls 2.73 -> 1.92 ms.
 // ------------------------------------------------------------------------------------------
 constexpr int kListThreads = 1024;                 // most threads of a block; one block per SM
 constexpr size_t kListSmemMax = 200 * 1024;        // shared memory a block may spend on its entries
